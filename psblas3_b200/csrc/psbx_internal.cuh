@@ -416,6 +416,7 @@ struct HllView {
   double *wpart;
   unsigned *wticket;
   const int *wcbase;
+  int entries;           // stored entries, padding included
 };
 
 struct HllViewF {  // FP32 values, FP32 x
@@ -432,6 +433,7 @@ struct EllView {
   const int *ja;
   const int *irn;
   int rows, pitch, base;
+  int entries;           // stored entries, padding included
 };
 
 struct EllViewF {  // FP32 values, FP32 x
@@ -446,6 +448,7 @@ struct CsrView {
   const int *ja;
   const int *irp;
   int rows, base;
+  int entries;
 };
 
 // HLL with the reference's GPU hack size (32 = warp size,

@@ -26,28 +26,11 @@
 // (e.g. x = alpha*p + x; r = -alpha*q + r; p = z + beta*p) with rounded
 // multiplies and adds, so they match the CPU path bit for bit given the same
 // scalars; only the reduction order differs.
-#include "psbx_internal.cuh"
+#include "psbx_krylov.cuh"
 
 #include <string.h>
 #include <strings.h>
 #include <vector>
-
-// ST_XUPD: a GMRES cycle ended (converged or nl steps); x is updated next.
-enum { ST_RUN = 0, ST_DONE = 1, ST_BREAK = 2, ST_XUPD = 3 };
-
-struct KState {
-  double rho, rho_old, sigma, alpha, beta, omega, tau;
-  double bn2, bni, ani, r0n2;
-  double errnum, errden, eps;
-  double gamma, delta, theta1, theta2;  // FCG
-  double scal;                          // GMRES: scale of the next basis vector
-  int itmax, istop;
-  int it, itx;
-  int status;
-  int r0set;
-  int first;                            // FCG: first step after a restart
-  int gm_m, gm_conv;                    // GMRES: basis vectors in the x update; converged
-};
 
 #define KT 256
 #define KLANES 4
@@ -1586,9 +1569,25 @@ static KCache *kc_slot(cudaStream_t st) {  // a free entry, else the least recen
   return lru;
 }
 
+// Systems in the one-kernel solver's range (psbx_persist.cu): their vectors
+// fit the SMs' shared memory.  Matrices with wide hacks stay with the
+// kernel-per-step driver, which sums the long rows over many blocks.
+static inline const HllView &persist_view(const HllView &A) { return A; }
+static inline const EllView &persist_view(const EllView &A) { return A; }
+static inline const CsrView &persist_view(const CsrView &A) { return A; }
+template <class View> static inline bool small_system(const View &A, bool bicg) {
+  return persist_fits(persist_view(A), bicg);
+}
+static inline bool small_system(const Hll32WView &, bool) { return false; }
+
 template <class View>
 static int solve(const View &A, bool bicg, const double *dinv, const double *b, double *x, int n,
                  psbx_SolverOptions *opt) {
+  if (small_system(A, bicg)) {
+    int ran = 0;
+    const int prc = persist_solve(persist_view(A), bicg, dinv, b, x, opt, &ran);
+    if (prc || ran) return prc;
+  }
   PsbxCtx &c = psbx_ctx();
   cudaStream_t st = c.stream;
   const int nvec = bicg ? 8 : 4;

@@ -55,6 +55,7 @@ HllView hll_view(const HllDevice *m) {
   v.wpart = wide ? m->wpart : nullptr;
   v.wticket = wide ? m->wticket : nullptr;
   v.wcbase = wide ? m->wcbase : nullptr;
+  v.entries = m->allocsize;
   return v;
 }
 
@@ -354,6 +355,7 @@ EllView ell_view(const EllDevice *m) {
   v.rows = m->rows;
   v.pitch = m->pitch;
   v.base = m->baseIndex;
+  v.entries = m->pitch * m->maxRowSize;
   return v;
 }
 
@@ -364,6 +366,7 @@ CsrView csr_view(const CsrDevice *m) {
   v.irp = m->irp;
   v.rows = m->m;
   v.base = m->baseIndex;
+  v.entries = m->nz;
   return v;
 }
 
