@@ -28,9 +28,9 @@
 // indices) with 1-based local columns, and K interleaved vectors
 // v[row*K + j].  Work is cut in tiles of rows of one system (tile_plan);
 // block b takes tiles b, b + grid, b + 2 grid, ... so the blocks in flight
-// work on a window of consecutive tiles (whose gathered vectors share L2).  A tile's partial sums go to
-// part[tile]; the block that completes the last tile of a system (per-system
-// ticket) adds that system's partials in tile order -- fixed order, so the
+// work on a window of consecutive tiles (whose gathered vectors share L2).  A
+// tile's partial sums go to part[tile]; the block whose tickets complete a
+// system adds that system's partials in tile order -- fixed order, so the
 // result does not depend on scheduling -- and advances the system's phase.
 // Every kernel only touches systems in its own phase; a graph of ITERS x 6
 // kernels is replayed and the host looks at the phases once per replay.
@@ -44,12 +44,28 @@ namespace {
 
 enum Phase { PH_IDLE = 0, PH_RESID = 1, PH_INIT = 2, PH_INNER = 3, PH_XUPD = 4, PH_DONE = 5 };
 enum { BT = 256, ITERS = 8, MAXK = 8, LONG_ROW = 64 };
-// Thread-per-row tile bounds (rows, stored entries): one right-hand side
-// runs fastest with 4096 / 32K (7-point 111^3: 17.8 ms per solve against
-// 19.7 with 2048 / 16K), eight with 2048 / 16K (their SpMV carries 8 sums
-// per row: 534 against 635 us per launch on C4).
-__host__ __device__ constexpr int tile_rows(int K) { return K == 1 ? 4096 : 2048; }
-__host__ __device__ constexpr int tile_nnz(int K) { return K == 1 ? 32768 : 16384; }
+// Thread-per-row tile bounds (rows, stored entries).  Fine tiles fill the
+// last round of the grid and small batches; what a tile costs beyond its rows
+// is small (run_tiles).  32 serving-like systems with one right-hand side:
+// 86 ms a solve of all with 4096 rows, 69 with 2048, 60 with 1024, 66 with 512;
+// 128 anisotropic systems with eight: 390 ms with 2048, 320 with 1024, 336
+// with 512 (16 of them: 91, 61, 62).
+__host__ __device__ constexpr int tile_rows(int /*K*/) { return 1024; }
+__host__ __device__ constexpr int tile_nnz(int K) { return 8 * tile_rows(K); }
+
+// Eight right-hand sides are spread over L = 2 neighbouring lanes of H = 4
+// each: a row of a vector is then one 16-byte (FP32) access per lane, a warp
+// moves 512 contiguous bytes per instruction, a gathered row is one 32-byte
+// sector, and a thread carries 4 sums instead of 8.
+template <int K> struct Lay {
+  static constexpr int H = K == 8 ? 4 : 1;
+  static constexpr int L = K / H;
+  static constexpr int R = BT / L;  // rows per pass of the block
+};
+// Entries of a row that the products load together.
+template <int K, class VT> struct SpmvRow {
+  static constexpr int U = K == 1 || sizeof(VT) == 4 ? 8 : 4;
+};
 
 struct BSys {                 // read-only for the kernels
   const double *val64;
@@ -57,7 +73,7 @@ struct BSys {                 // read-only for the kernels
   const int *ja, *irn, *hkoffs;
   const double *b;
   double *x, *r64;
-  void *r32, *z, *p, *q, *d;  // inner vectors, of the engine's inner type (float, or double)
+  void *r32, *p, *q, *d;      // inner vectors, of the engine's inner type (float, or double)
   const void *dinv;           // inverse diagonal, inner type
   int rows, sol0, tile0, ntiles;
 };
@@ -110,7 +126,7 @@ struct BCtl {                 // read by every kernel at launch; lets the tile
 };
 
 struct Eng {
-  int K = 1, max_sys = 0, max_tiles = 0, grid = 0;
+  int K = 1, max_sys = 0, max_tiles = 0, sms = 0;
   int fp64 = 0;               // inner iterations in FP64 (the batched FP64 comparison) instead of FP32
   BSys *d_sys = nullptr;
   BState *d_state = nullptr;
@@ -141,22 +157,22 @@ struct Eng {
 };
 
 // --------------------------------------------------------------- helpers
-// Occupancy targets (blocks of BT threads per SM).  The K = 1 kernels are
-// latency-bound streams over short rows: the SpMV and the short vector
-// kernels want every warp slot (8 blocks, <= 32 registers); the update keeps
-// 4 rows of loads in flight per thread instead (4 blocks, no spills), which
-// measured faster than 1 row per thread at 8 blocks.  The 8-rhs kernels carry
-// 8 accumulators per row; their SpMV runs 4 blocks per SM even though that
-// spills a few registers: on the 512 anisotropic systems 534 us, against
-// 672 us at 2 blocks, 712 us at 3, 655 us at 3 blocks with 4 entries per
-// load group, and 750-850 us when the 8 sums are formed as two halves of 4.
+// Occupancy targets (blocks of BT threads per SM): the most warps that hold
+// their loads in registers.  A spilled load waits for memory at once: the
+// 8-rhs SpMV at 5 blocks took 424 ms a batch against 320 at 4, the 1-rhs one
+// 69 ms at 8 blocks against 60 at 6.
 template <int K> struct Occ {
-  static constexpr int blocks = K == 1 ? 8 : 2;
-  static constexpr int spmv_blocks = K == 1 ? 8 : 4;
-  static constexpr int update_blocks = K == 1 ? 4 : 2;
-  static constexpr int resid_blocks = K == 1 ? 4 : 2;
+  static constexpr int blocks = K == 1 ? 6 : 4;
+  static constexpr int spmv_blocks = K == 1 ? 6 : 4;
+  static constexpr int update_blocks = 4;
+  static constexpr int resid_blocks = K == 1 ? 4 : 3;
 };
 
+// acc + a*b: the product of two floats is exact in FP64, so one fused
+// multiply-add rounds as the multiply and the add do; FP64 factors are
+// multiplied and added.
+__device__ __forceinline__ double mac(double acc, float a, float b) { return __fma_rn((double)a, (double)b, acc); }
+__device__ __forceinline__ double mac(double acc, double a, double b) { return radd(acc, rmul(a, b)); }
 
 // A kernel whose phase no system is in returns after one load (instead of
 // walking the tile table); the finalisers move systems between phases and
@@ -268,51 +284,37 @@ __device__ __forceinline__ void st_row(double *p, const double (&v)[K]) {
   }
 }
 
-// Row sums of one HLL-32 row for K interleaved vectors, entries in order.
-template <class VT, class XT, int K>
-__device__ __forceinline__ void row_multi(const VT *__restrict__ val, const int *__restrict__ ja, RowRef rr,
-                                          const XT *__restrict__ x, double (&acc)[K]) {
-  const VT *vp = val + rr.off;
-  const int *jp = ja + rr.off;
-  const int n = rr.n;
+// Entries j .. j + U - 1 of an HLL-32 row (those within it; FULL: all are),
+// loads only.
+template <class VT, int U, bool FULL>
+__device__ __forceinline__ void ld_entries(const VT *__restrict__ val, const int *__restrict__ ja, RowRef rr, int j,
+                                           int (&c)[U], VT (&v)[U]) {
 #pragma unroll
-  for (int k = 0; k < K; k++) acc[k] = 0.0;
-  constexpr int U = K == 1 ? 8 : 2;
-  int j = 0;
-  for (; j + U <= n; j += U) {
-    int c[U];
-    VT v[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      c[u] = ld_stream(jp + (j + u) * 32) - 1;
-      v[u] = ld_stream(vp + (j + u) * 32);
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      XT xv[K];
-      ld_row_ro<K>(x + (size_t)c[u] * K, xv);
-#pragma unroll
-      for (int k = 0; k < K; k++) acc[k] = radd(acc[k], rmul((double)v[u], (double)xv[k]));
-    }
+  for (int u = 0; u < U; u++) {
+    const bool ok = FULL || j + u < rr.n;
+    c[u] = ok ? ld_stream(ja + rr.off + (j + u) * 32) - 1 : 0;
+    v[u] = ok ? ld_stream(val + rr.off + (j + u) * 32) : VT(0);
   }
-  if (j < n) {  // the tail as one predicated group: its loads overlap
-    int c[U];
-    VT v[U];
+}
+
+// Adds those entries' products to the sums of the lane's H right-hand sides
+// (x at the lane's first one), in order.
+template <class VT, class XT, int K, int U, bool FULL>
+__device__ __forceinline__ void add_entries(RowRef rr, int j, const int (&c)[U], const VT (&v)[U],
+                                            const XT *__restrict__ x, double (&acc)[Lay<K>::H]) {
+  constexpr int H = Lay<K>::H, G = H > 1 && U > 4 ? 4 : U;  // gathers in flight
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const bool ok = j + u < n;
-      c[u] = ok ? ld_stream(jp + (j + u) * 32) - 1 : 0;
-      v[u] = ok ? ld_stream(vp + (j + u) * 32) : VT(0);
-    }
+  for (int g = 0; g < U; g += G) {
+    XT xv[G][H];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      if (j + u < n) {
-        XT xv[K];
-        ld_row_ro<K>(x + (size_t)c[u] * K, xv);
+    for (int u = 0; u < G; u++)
+      if (FULL || j + g + u < rr.n) ld_row_ro<H>(x + (size_t)c[g + u] * K, xv[u]);
 #pragma unroll
-        for (int k = 0; k < K; k++) acc[k] = radd(acc[k], rmul((double)v[u], (double)xv[k]));
+    for (int u = 0; u < G; u++)
+      if (FULL || j + g + u < rr.n) {
+#pragma unroll
+        for (int k = 0; k < H; k++) acc[k] = mac(acc[k], v[g + u], xv[u][k]);
       }
-    }
   }
 }
 
@@ -325,163 +327,282 @@ __device__ __forceinline__ void row_multi(const VT *__restrict__ val, const int 
 // 32 partial sums of a row are added in column-phase order; thread i < nrows
 // returns row i's sums.  Every thread of the block must call it.
 static_assert(BT / 32 == 8, "a long-row tile holds BT/32 = 8 rows");
-template <class VT, class XT, int K>
+template <class VT, class XT>
 __device__ __forceinline__ bool rows_by_block(const BSys &S, const BTile &T, const VT *__restrict__ val,
-                                              const XT *__restrict__ x, double (&out)[K]) {
-  __shared__ double red[K * BT];
+                                              const XT *__restrict__ x, double (&out)[1]) {
+  __shared__ double red[BT];
   const int i = threadIdx.x & 7, c0 = threadIdx.x >> 3;
-  double acc[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) acc[k] = 0.0;
+  double acc = 0.0;
   if (i < T.nrows) {
     const RowRef rr = row_ref(S.hkoffs, S.irn, T.row0 + i);
-    constexpr int W = K == 1 ? 8 : 2;
+    constexpr int W = 8;
     for (int j0 = c0; j0 < rr.n; j0 += 32 * W) {
       int c[W];
-      double v[W];
+      VT v[W];
 #pragma unroll
       for (int u = 0; u < W; u++) {
         const int j = j0 + 32 * u;
         const bool ok = j < rr.n;
         c[u] = ok ? ld_stream(S.ja + rr.off + j * 32) - 1 : 0;
-        v[u] = ok ? (double)ld_stream(val + rr.off + j * 32) : 0.0;
+        v[u] = ok ? ld_stream(val + rr.off + j * 32) : VT(0);
       }
 #pragma unroll
-      for (int u = 0; u < W; u++) {
-        if (j0 + 32 * u < rr.n) {
-          XT xv[K];
-          ld_row_ro<K>(x + (size_t)c[u] * K, xv);
-#pragma unroll
-          for (int k = 0; k < K; k++) acc[k] = radd(acc[k], rmul(v[u], (double)xv[k]));
-        }
-      }
+      for (int u = 0; u < W; u++)
+        if (j0 + 32 * u < rr.n) acc = mac(acc, v[u], __ldg(x + c[u]));
     }
   }
-#pragma unroll
-  for (int k = 0; k < K; k++) red[k * BT + threadIdx.x] = acc[k];
+  red[threadIdx.x] = acc;
   __syncthreads();
   const bool mine = threadIdx.x < T.nrows;
   if (mine) {
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      double t = 0.0;
-      for (int c = 0; c < BT / 8; c++) t = radd(t, red[k * BT + c * 8 + threadIdx.x]);
-      out[k] = t;
-    }
+    double t = 0.0;
+    for (int c = 0; c < BT / 8; c++) t = radd(t, red[c * 8 + threadIdx.x]);
+    out[0] = t;
   }
   __syncthreads();  // red is reused by the next tile
   return mine;
 }
 
 // One long row summed by a whole warp (the 8-right-hand-side kernels, where
-// the block-wide sums below cost registers): lane l takes entries l, l+32,
-// ...; a fixed shuffle tree combines them; the result is valid in every lane.
+// the block-wide sums below cost registers): lane pair l takes entries l,
+// l+16, ...; a fixed shuffle tree combines them; the result is valid in every
+// lane (each for its 4 right-hand sides).
 template <class VT, class XT, int K>
 __device__ __forceinline__ void row_multi_warp(const VT *__restrict__ val, const int *__restrict__ ja, RowRef rr,
-                                               const XT *__restrict__ x, double (&acc)[K]) {
-  const int lane = threadIdx.x & 31;
+                                               const XT *__restrict__ x, double (&acc)[Lay<K>::H]) {
+  constexpr int H = Lay<K>::H, L = Lay<K>::L, P = 32 / L;
+  const int lane = (threadIdx.x & 31) / L;
 #pragma unroll
-  for (int k = 0; k < K; k++) acc[k] = 0.0;
-  // a lane's entries lane, lane+32, ... in order, W of them per round with
+  for (int k = 0; k < H; k++) acc[k] = 0.0;
+  // a lane's entries lane, lane+P, ... in order, W of them per round with
   // all their loads issued before the gathers
-  constexpr int W = K == 1 ? 8 : 2;
-  for (int j0 = lane; j0 < rr.n; j0 += 32 * W) {
+  constexpr int W = 4;
+  for (int j0 = lane; j0 < rr.n; j0 += P * W) {
     int c[W];
-    double v[W];
+    VT v[W];
 #pragma unroll
     for (int u = 0; u < W; u++) {
-      const int j = j0 + 32 * u;
+      const int j = j0 + P * u;
       const bool ok = j < rr.n;
       c[u] = ok ? ld_stream(ja + rr.off + j * 32) - 1 : 0;
-      v[u] = ok ? (double)ld_stream(val + rr.off + j * 32) : 0.0;
+      v[u] = ok ? ld_stream(val + rr.off + j * 32) : VT(0);
     }
 #pragma unroll
     for (int u = 0; u < W; u++) {
-      if (j0 + 32 * u < rr.n) {
-        XT xv[K];
-        ld_row_ro<K>(x + (size_t)c[u] * K, xv);
+      if (j0 + P * u < rr.n) {
+        XT xv[H];
+        ld_row_ro<H>(x + (size_t)c[u] * K, xv);
 #pragma unroll
-        for (int k = 0; k < K; k++) acc[k] = radd(acc[k], rmul(v[u], (double)xv[k]));
+        for (int k = 0; k < H; k++) acc[k] = mac(acc[k], v[u], xv[k]);
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < K; k++)
+  for (int k = 0; k < H; k++)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc[k] = radd(acc[k], __shfl_xor_sync(0xffffffffu, acc[k], o));
+    for (int o = 16; o >= L; o >>= 1) acc[k] = radd(acc[k], __shfl_xor_sync(0xffffffffu, acc[k], o));
 }
 
-// Applies f(row, sums) to every row of a tile: thread-per-row tiles (kind 0)
-// walk rows threadIdx.x, +BT, ... with the next row's offset and length
-// loaded while the current row is summed; the rows of a long-row tile
-// (kind 1) are summed by the whole block and f is called by thread i for row
-// i (one right-hand side), or by a warp per row, f in lane 0 (8 of them).
+// Applies f(i, o, sums) to every row i of a tile, o the position of the lane's
+// right-hand sides of the row in an interleaved vector: thread-per-row tiles
+// (kind 0) walk rows R apart with the next row's offset and length loaded
+// while the current row is summed; the rows of a long-row tile (kind 1) are
+// summed by the whole block and f is called by
+// thread i for row i (one right-hand side), or by a warp per row, f in its
+// first L lanes (8 of them).
 template <class VT, class XT, int K, class F>
 __device__ __forceinline__ void tile_spmv(const BSys &S, const BTile &T, const VT *__restrict__ val,
                                           const XT *__restrict__ x, F &&f) {
+  constexpr int H = Lay<K>::H, L = Lay<K>::L;
+  const int q = (threadIdx.x % L) * H;
   if (T.kind == 1) {
     if constexpr (K == 1) {
-      double a[K];
-      if (rows_by_block<VT, XT, K>(S, T, val, x, a)) f(T.row0 + threadIdx.x, a);
+      double a[1];
+      if (rows_by_block(S, T, val, x, a)) f((int)threadIdx.x, (size_t)T.row0 + threadIdx.x, a);
     } else {
       for (int i = threadIdx.x >> 5; i < T.nrows; i += BT / 32) {
         const int r = T.row0 + i;
-        double a[K];
-        row_multi_warp<VT, XT, K>(val, S.ja, row_ref(S.hkoffs, S.irn, r), x, a);
-        if ((threadIdx.x & 31) == 0) f(r, a);
+        double a[H];
+        row_multi_warp<VT, XT, K>(val, S.ja, row_ref(S.hkoffs, S.irn, r), x + q, a);
+        if ((threadIdx.x & 31) < L) f(i, (size_t)r * K + q, a);
       }
     }
     return;
   }
-  int i = threadIdx.x;
-  RowRef cur = {0, 0};
-  if (i < T.nrows) cur = row_ref(S.hkoffs, S.irn, T.row0 + i);
-  for (; i < T.nrows; i += BT) {
-    RowRef nxt = {0, 0};
-    if (i + BT < T.nrows) nxt = row_ref(S.hkoffs, S.irn, T.row0 + i + BT);
-    double a[K];
-    row_multi<VT, XT, K>(val, S.ja, cur, x, a);
-    f(T.row0 + i, a);
+  constexpr int U = SpmvRow<K, VT>::U;
+  auto ref = [&](int i) { return i < T.nrows ? row_ref(S.hkoffs, S.irn, T.row0 + i) : RowRef{0, 0}; };
+  int i = threadIdx.x / L;
+  RowRef cur = ref(i);
+  for (; i < T.nrows; i += Lay<K>::R) {
+    const RowRef nxt = ref(i + Lay<K>::R);
+    double a[H];
+#pragma unroll
+    for (int k = 0; k < H; k++) a[k] = 0.0;
+    int j = 0;
+    for (; j + U <= cur.n; j += U) {
+      int c[U];
+      VT v[U];
+      ld_entries<VT, U, true>(val, S.ja, cur, j, c, v);
+      add_entries<VT, XT, K, U, true>(cur, j, c, v, x + q, a);
+    }
+    if (j < cur.n) {  // the tail as one predicated group: its loads overlap
+      int c[U];
+      VT v[U];
+      ld_entries<VT, U, false>(val, S.ja, cur, j, c, v);
+      add_entries<VT, XT, K, U, false>(cur, j, c, v, x + q, a);
+    }
+    f(i, (size_t)(T.row0 + i) * K + q, a);
     cur = nxt;
   }
 }
 
-// Block-reduce NS sums per rhs (K of each), publish the tile's partials,
-// take the system's ticket; returns true in the block that finalises.
-template <int K, int NS>
-__device__ __forceinline__ bool tile_publish(double (&v)[NS][K], double *part, int tile, BState *st, int ntiles,
-                                             double *smem /* >= 32*NS*K */) {
-#pragma unroll
-  for (int m = 0; m < NS; m++) {
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      double t = v[m][k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t = radd(t, __shfl_down_sync(0xffffffffu, t, o));
-      v[m][k] = t;
-    }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) {
+// NS sums over a tile's rows per rhs, in one order whatever K is, so that a
+// right-hand side gives the same bits alone and among eight: the terms of
+// rows c, c + 128, c + 256, ... in order, for each c < 128; 16 neighbouring c
+// in a tree; the 8 groups in order.  With eight right-hand sides those rows
+// are one thread's, which keeps its sums in registers; with one, a pass of the
+// block is two of these rows, and the terms go to shared memory first.
+enum { CLS = 128, GROUPS = CLS / 16 };
+template <int K, int NS> struct TileSums {
+  static constexpr int H = Lay<K>::H;
+  static_assert(K == 1 || Lay<K>::R == CLS, "a thread's rows are CLS apart");
+  struct Shared {
+    double term[K == 1 ? NS : 1][K == 1 ? tile_rows(K) : 1];
+    double group[2][NS * K][GROUPS];  // two tiles in turn
+  };
+  Shared &sh;
+  double v[NS][H];
+  __device__ __forceinline__ explicit TileSums(Shared &s) : sh(s) {
 #pragma unroll
     for (int m = 0; m < NS; m++)
 #pragma unroll
-      for (int k = 0; k < K; k++) smem[(m * K + k) * 32 + warp] = v[m][k];
+      for (int k = 0; k < H; k++) v[m][k] = 0.0;
   }
-  __syncthreads();
-  if (threadIdx.x < NS * K) {
-    double s = 0.0;
-    for (int w = 0; w < BT / 32; w++) s = radd(s, smem[threadIdx.x * 32 + w]);
-    part[(size_t)tile * (2 * MAXK) + threadIdx.x] = s;
+  // sum m of the lane's rhs k takes the product a*b of row i of the tile
+  template <class T> __device__ __forceinline__ void add(int i, int m, int k, T a, T b) {
+    if constexpr (K == 1) sh.term[m][i] = rmul((double)a, (double)b);  // (exact for floats)
+    else v[m][k] = mac(v[m][k], a, b);
   }
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == (unsigned)(ntiles - 1);
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
+  // the sums of rows 0 .. n-1 into part[tile]
+  __device__ __forceinline__ void store(int n, int j, double *part, int tile) {
+    const int lane = threadIdx.x & 31;
+    double (*group)[GROUPS] = sh.group[j & 1];
+    if constexpr (K == 1) {
+      __syncthreads();
+      const int c = threadIdx.x % CLS, m = threadIdx.x / CLS;
+      if (m < NS) {  // whole warps
+        double t = 0.0;
+#pragma unroll
+        for (int u = 0; u < tile_rows(K) / CLS; u++)
+          if (c + u * CLS < n) t = radd(t, sh.term[m][c + u * CLS]);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t = radd(t, __shfl_down_sync(0xffffffffu, t, o));
+        if (lane % 16 == 0) group[m][c / 16] = t;
+      }
+    } else {
+      constexpr int L = Lay<K>::L;
+#pragma unroll
+      for (int m = 0; m < NS; m++)
+#pragma unroll
+        for (int k = 0; k < H; k++) {
+          double t = v[m][k];
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) t = radd(t, __shfl_down_sync(0xffffffffu, t, o * L));
+          if (lane < L) group[m * K + lane * H + k][threadIdx.x >> 5] = t;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < NS * K) {
+      double s = 0.0;
+#pragma unroll
+      for (int g = 0; g < GROUPS; g++) s = radd(s, group[threadIdx.x][g]);
+      part[(size_t)tile * (2 * MAXK) + threadIdx.x] = s;
+    }
+  }
+};
+static_assert(2 * CLS <= BT && BT / 32 == GROUPS, "one thread per class and sum; a warp is a group of lane pairs");
+
+// The tiles of one block in one kernel: CH at a time, the descriptors of those
+// whose system is in the kernel's phase, their systems, and the scalars of
+// their right-hand sides are brought to shared memory together, then the
+// tiles are worked through without waiting for any of it; the systems'
+// tickets are taken after the last one, behind one fence.  Per tile, those
+// four dependent reads and the fence and ticket were about 4 us, as much as
+// the work of 512 rows.
+enum { CH = 32 };
+enum { SC_ACTIVE = 1, SC_FIRST = 2, SC_DONE = 4 };
+template <int K> struct TileChunk {
+  BTile t[CH];
+  int idx[CH];          // tile numbers
+  int n;
+  unsigned fin;         // tiles whose ticket was their system's last
+  BSys s[CH];
+  double alpha[CH][K];
+  double beta[CH][K];   // beta in PH_INNER, else the scale
+  int flags[CH][K];
+};
+
+// body(C, j, S, T): tile j of the chunk; fin(S, state): the system's last tile
+// is done (its partials are visible), called by the whole block.
+template <int K, int PH, bool SCALARS, bool TICKET, class Body, class Fin>
+__device__ __forceinline__ void run_tiles(const BSys *__restrict__ sys, BState *state, const BSol *sol,
+                                          const BCtl *ctl, Body &&body, Fin &&fin) {
+  __shared__ TileChunk<K> C;
+  static_assert(sizeof(BSys) % 8 == 0, "copied in 8-byte words");
+  constexpr int W = sizeof(BSys) / 8;
+  if (phase_idle(ctl, PH)) return;
+  const BTile *__restrict__ tiles = ctl->tiles;
+  const int ntiles = ctl->ntiles;
+  for (int base = blockIdx.x; base < ntiles; base += CH * gridDim.x) {
+    if (threadIdx.x < 32) {
+      const int t = base + threadIdx.x * gridDim.x;
+      BTile T = {0, 0, 0, 0};
+      if (t < ntiles) T = tiles[t];
+      const bool ok = t < ntiles && state[T.sys].phase == PH;
+      const unsigned m = __ballot_sync(0xffffffffu, ok);
+      const int pos = __popc(m & ((1u << threadIdx.x) - 1));
+      if (ok) {
+        C.t[pos] = T;
+        C.idx[pos] = t;
+      }
+      if (threadIdx.x == 0) C.n = __popc(m);
+    }
+    __syncthreads();
+    const int n = C.n;
+    for (int w = threadIdx.x; w < n * W; w += BT)
+      ((unsigned long long *)&C.s[w / W])[w % W] = ((const unsigned long long *)(sys + C.t[w / W].sys))[w % W];
+    if (SCALARS) {
+      for (int w = threadIdx.x; w < n * K; w += BT) {
+        const int j = w / K, k = w % K;
+        const BSol *so = sol + (size_t)C.t[j].sys * K + k;
+        C.alpha[j][k] = so->alpha;
+        C.beta[j][k] = PH == PH_INNER ? so->beta : so->scale;
+        C.flags[j][k] = (so->active ? SC_ACTIVE : 0) | (so->it == 1 ? SC_FIRST : 0) | (so->done ? SC_DONE : 0);
+      }
+    }
+    __syncthreads();
+    for (int j = 0; j < n; j++) body(C, j, C.s[j], C.t[j]);
+    if (TICKET && n > 0) {
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        bool last = false;
+        if ((int)threadIdx.x < n)
+          last = atomicAdd(&state[C.t[threadIdx.x].sys].ticket, 1u) == (unsigned)(C.s[threadIdx.x].ntiles - 1);
+        const unsigned m = __ballot_sync(0xffffffffu, last);
+        if (threadIdx.x == 0) C.fin = m;
+      }
+      __syncthreads();
+      unsigned m = C.fin;
+      if (m) __threadfence();
+      for (; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        fin(C.s[j], state + C.t[j].sys);
+        __syncthreads();
+      }
+    }
+    __syncthreads();  // C is refilled
+  }
 }
 
 // Totals of the system's tile partials for NV values (all threads of the
@@ -491,7 +612,7 @@ __device__ __forceinline__ bool tile_publish(double (&v)[NS][K], double *part, i
 // Results in tot[0..NV).
 template <int NV>
 __device__ __forceinline__ void sys_totals(const double *part, int tile0, int ntiles, double *tot,
-                                           double *scratch /* 32*NV */) {
+                                           double *scratch /* 8*NV */) {
   double v[NV];
 #pragma unroll
   for (int m = 0; m < NV; m++) v[m] = 0.0;
@@ -509,12 +630,12 @@ __device__ __forceinline__ void sys_totals(const double *part, int tile0, int nt
   __syncthreads();
   if (lane == 0) {
 #pragma unroll
-    for (int m = 0; m < NV; m++) scratch[m * 32 + warp] = v[m];
+    for (int m = 0; m < NV; m++) scratch[m * 8 + warp] = v[m];
   }
   __syncthreads();
   if (threadIdx.x < NV) {
     double s = 0.0;
-    for (int w = 0; w < BT / 32; w++) s = radd(s, scratch[threadIdx.x * 32 + w]);
+    for (int w = 0; w < BT / 32; w++) s = radd(s, scratch[threadIdx.x * 8 + w]);
     tot[threadIdx.x] = s;
   }
   __syncthreads();
@@ -526,33 +647,30 @@ __device__ __forceinline__ void sys_totals(const double *part, int tile0, int nt
 template <int K>
 __global__ void __launch_bounds__(BT, Occ<K>::resid_blocks) kb_resid(const BSys *__restrict__ sys, BState *state,
                                                                      BSol *sol, const BCtl *ctl) {
-  __shared__ double sm[32 * 2 * MAXK];
-  if (phase_idle(ctl, PH_RESID)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
+  constexpr int H = Lay<K>::H;
+  __shared__ typename TileSums<K, 2>::Shared sums;
+  __shared__ double sm[8 * 2 * MAXK];
   double *part = ctl->part;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    BState *st = state + T.sys;
-    if (st->phase != PH_RESID) continue;
-    const BSys &S = sys[T.sys];
-    double v[2][K];
+  run_tiles<K, PH_RESID, false, true>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        const double *__restrict__ b = S.b;
+        double *__restrict__ r64 = S.r64;
+        TileSums<K, 2> acc(sums);
+        tile_spmv<double, double, K>(S, T, S.val64, S.x, [&](int i, size_t o, const double (&ax)[H]) {
+          double bb[H], rr[H];
+          ld_row<H>(b + o, bb);
 #pragma unroll
-    for (int k = 0; k < K; k++) v[0][k] = v[1][k] = 0.0;
-    const double *__restrict__ b = S.b;
-    double *__restrict__ r64 = S.r64;
-    tile_spmv<double, double, K>(S, T, S.val64, S.x, [&](int r, const double (&ax)[K]) {
-      double bb[K], rr[K];
-      ld_row<K>(b + (size_t)r * K, bb);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        rr[k] = radd(bb[k], -ax[k]);
-        v[0][k] = radd(v[0][k], rmul(rr[k], rr[k]));
-        v[1][k] = radd(v[1][k], rmul(bb[k], bb[k]));
-      }
-      st_row<K>(r64 + (size_t)r * K, rr);
-    });
-    if (tile_publish<K, 2>(v, part, t, st, S.ntiles, sm)) {
+          for (int k = 0; k < H; k++) {
+            rr[k] = radd(bb[k], -ax[k]);
+            acc.add(i, 0, k, rr[k], rr[k]);
+            acc.add(i, 1, k, bb[k], bb[k]);
+          }
+          st_row<H>(r64 + o, rr);
+        });
+        acc.store(T.nrows, j, part, C.idx[j]);
+      },
+      [&](const BSys &S, BState *st) {
       __shared__ double tot[2 * K];
       sys_totals<2 * K>(part, S.tile0, S.ntiles, tot, sm);
       if (threadIdx.x < K) {
@@ -590,72 +708,65 @@ __global__ void __launch_bounds__(BT, Occ<K>::resid_blocks) kb_resid(const BSys 
         st->done_flag = all;
         st->ticket = 0;
       }
-    }
-  }
+      });
 }
 
-// PH_INIT: r32 = r/scale, z = D r32, d = 0; rho = (r32, z).
+// PH_INIT: r32 = r/scale, d = 0; rho = (r32, D r32).
 template <int K, class TI>
 __global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_init(const BSys *__restrict__ sys, BState *state,
                                                               BSol *sol, const BCtl *ctl) {
-  constexpr int RB = K == 1 ? 2 : 1;  // rows per thread whose loads are in flight together
-  __shared__ double sm[32 * 2 * MAXK];
-  if (phase_idle(ctl, PH_INIT)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
+  constexpr int H = Lay<K>::H, L = Lay<K>::L, R = Lay<K>::R;
+  constexpr int RB = 2;  // rows per thread whose loads are in flight together
+  __shared__ typename TileSums<K, 1>::Shared sums;
+  __shared__ double sm[8 * 2 * MAXK];
   double *part = ctl->part;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    BState *st = state + T.sys;
-    if (st->phase != PH_INIT) continue;
-    const BSys &S = sys[T.sys];
-    double inv[K];
-    bool live[K];
+  const int q = (threadIdx.x % L) * H;
+  run_tiles<K, PH_INIT, true, true>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        double inv[H];
+        bool live[H];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const BSol *so = sol + S.sol0 + k;
-      live[k] = so->done == 0;
-      inv[k] = live[k] ? 1.0 / so->scale : 0.0;
-    }
-    const double *__restrict__ r64 = S.r64;
-    const TI *__restrict__ dinv = (const TI *)S.dinv;
-    TI *__restrict__ r32 = (TI *)S.r32;
-    TI *__restrict__ z = (TI *)S.z;
-    TI *__restrict__ d = (TI *)S.d;
-    double v[1][K];
-#pragma unroll
-    for (int k = 0; k < K; k++) v[0][k] = 0.0;
-    for (int i0 = threadIdx.x; i0 < T.nrows; i0 += RB * BT) {
-      double rv64[RB][K];
-      TI dg[RB];
-#pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        const size_t r = (size_t)T.row0 + i;
-        if (i < T.nrows) {
-          dg[u] = dinv[r];
-          ld_row<K>(r64 + r * K, rv64[u]);
+        for (int k = 0; k < H; k++) {
+          live[k] = !(C.flags[j][q + k] & SC_DONE);
+          inv[k] = live[k] ? 1.0 / C.beta[j][q + k] : 0.0;
         }
-      }
+        const double *__restrict__ r64 = S.r64;
+        const TI *__restrict__ dinv = (const TI *)S.dinv;
+        TI *__restrict__ r32 = (TI *)S.r32;
+        TI *__restrict__ d = (TI *)S.d;
+        TileSums<K, 1> acc(sums);
+        for (int i0 = threadIdx.x / L; i0 < T.nrows; i0 += RB * R) {
+          double rv64[RB][H];
+          TI dg[RB];
 #pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        if (i >= T.nrows) continue;
-        const size_t r = (size_t)T.row0 + i;
-        TI rv[K], zv[K], dz[K];
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            const size_t r = (size_t)T.row0 + i;
+            if (i < T.nrows) {
+              dg[u] = dinv[r];
+              ld_row<H>(r64 + r * K + q, rv64[u]);
+            }
+          }
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-          rv[k] = live[k] ? (TI)rmul(rv64[u][k], inv[k]) : TI(0);
-          zv[k] = rmul(dg[u], rv[k]);
-          dz[k] = TI(0);
-          v[0][k] = radd(v[0][k], rmul((double)rv[k], (double)zv[k]));
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            if (i >= T.nrows) continue;
+            const size_t o = ((size_t)T.row0 + i) * K + q;
+            TI rv[H], dz[H];
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+              rv[k] = live[k] ? (TI)rmul(rv64[u][k], inv[k]) : TI(0);
+              dz[k] = TI(0);
+              acc.add(i, 0, k, rv[k], rmul(dg[u], rv[k]));
+            }
+            st_row<H>(r32 + o, rv);
+            st_row<H>(d + o, dz);
+          }
         }
-        st_row<K>(r32 + r * K, rv);
-        st_row<K>(z + r * K, zv);
-        st_row<K>(d + r * K, dz);
-      }
-    }
-    if (tile_publish<K, 1>(v, part, t, st, S.ntiles, sm)) {
+        acc.store(T.nrows, j, part, C.idx[j]);
+      },
+      [&](const BSys &S, BState *st) {
       __shared__ double tot[K];
       sys_totals<K>(part, S.tile0, S.ntiles, tot, sm);
       if (threadIdx.x < K) {
@@ -675,6 +786,7 @@ __global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_init(const BSys *__rest
           so->rho = rho;
           so->active = so->rho > 0.0 ? 1 : 0;
         }
+        so->alpha = 0.0;  // no step pending
       }
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -682,100 +794,111 @@ __global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_init(const BSys *__rest
         st->outer += 1;
         st->ticket = 0;
       }
-    }
-  }
+      });
 }
 
-// PH_INNER: p = z (it == 1) or p = z + beta p, for active rhs.
+// PH_INNER: d += alpha p, the last iteration's step (p is read here anyway,
+// so the update kernel need not read it; alpha is 0 when no step is pending)
+// ; p = z (it == 1) or p = z + beta p, for active rhs, z = D r formed here
+// instead of being stored: 372 bytes a row and iteration with 8 right-hand
+// sides and 5-entry rows, against 432 with z and d in the update.
 template <int K, class TI>
-__global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_p(const BSys *__restrict__ sys, const BState *state,
+__global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_p(const BSys *__restrict__ sys, BState *state,
                                                            const BSol *sol, const BCtl *ctl) {
-  constexpr int RB = K == 1 ? 4 : 1;
-  if (phase_idle(ctl, PH_INNER)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    if (state[T.sys].phase != PH_INNER) continue;
-    const BSys &S = sys[T.sys];
-    TI beta[K];
-    bool act[K], first[K];
+  constexpr int H = Lay<K>::H, L = Lay<K>::L, R = Lay<K>::R;
+  constexpr int RB = (K == 1 ? 4 : 2) / (sizeof(TI) == 8 ? 2 : 1);
+  const int q = (threadIdx.x % L) * H;
+  run_tiles<K, PH_INNER, true, false>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        TI beta[H], alpha[H];
+        bool act[H], first[H];
+        // p of a stopped rhs keeps its value; it is read only when some rhs
+        // is past its first inner iteration or stopped
+        bool any_act = false, step = false, need_p = false;
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const BSol *so = sol + S.sol0 + k;
-      act[k] = so->active;
-      first[k] = so->it == 1;
-      beta[k] = (TI)so->beta;
-    }
-    const TI *__restrict__ z = (const TI *)S.z;
-    TI *__restrict__ p = (TI *)S.p;
-    // p of a stopped rhs keeps its value; it is read only when some rhs
-    // is past its first inner iteration or stopped
-    bool any_act = false, need_p = false;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      any_act |= act[k];
-      need_p |= !act[k] || !first[k];
-    }
-    if (!any_act) continue;
-    for (int i0 = threadIdx.x; i0 < T.nrows; i0 += RB * BT) {
-      TI zv[RB][K], pv[RB][K];
-#pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        const size_t o = ((size_t)T.row0 + i) * K;
-#pragma unroll
-        for (int k = 0; k < K; k++) pv[u][k] = TI(0);
-        if (i < T.nrows) {
-          ld_row<K>(z + o, zv[u]);
-          if (need_p) ld_row<K>(p + o, pv[u]);
+        for (int k = 0; k < H; k++) {
+          const int f = C.flags[j][q + k];
+          act[k] = f & SC_ACTIVE;
+          first[k] = f & SC_FIRST;
+          beta[k] = (TI)C.beta[j][q + k];
+          alpha[k] = (TI)C.alpha[j][q + k];
+          any_act |= act[k];
+          step |= alpha[k] != TI(0);
+          need_p |= !act[k] || !first[k];
         }
-      }
+        need_p |= step;
+        if (!any_act && !step) return;
+        const TI *__restrict__ r32 = (const TI *)S.r32;
+        const TI *__restrict__ dinv = (const TI *)S.dinv;
+        TI *__restrict__ p = (TI *)S.p;
+        TI *__restrict__ d = (TI *)S.d;
+        for (int i0 = threadIdx.x / L; i0 < T.nrows; i0 += RB * R) {
+          TI rv[RB][H], pv[RB][H], dv[RB][H], dg[RB];
 #pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        if (i >= T.nrows) continue;
-        const size_t o = ((size_t)T.row0 + i) * K;
-        TI pn[K];
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            const size_t o = ((size_t)T.row0 + i) * K + q;
 #pragma unroll
-        for (int k = 0; k < K; k++)
-          pn[k] = !act[k] ? pv[u][k] : first[k] ? zv[u][k] : radd(zv[u][k], rmul(beta[k], pv[u][k]));
-        st_row<K>(p + o, pn);
-      }
-    }
-  }
+            for (int k = 0; k < H; k++) pv[u][k] = TI(0);
+            if (i < T.nrows) {
+              dg[u] = dinv[T.row0 + i];
+              ld_row<H>(r32 + o, rv[u]);
+              if (need_p) ld_row<H>(p + o, pv[u]);
+              if (step) ld_row<H>(d + o, dv[u]);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            if (i >= T.nrows) continue;
+            const size_t o = ((size_t)T.row0 + i) * K + q;
+            if (step) {
+#pragma unroll
+              for (int k = 0; k < H; k++)
+                if (alpha[k] != TI(0)) dv[u][k] = radd(dv[u][k], rmul(alpha[k], pv[u][k]));
+              st_row<H>(d + o, dv[u]);
+            }
+            TI pn[H];
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+              const TI z = rmul(dg[u], rv[u][k]);
+              pn[k] = !act[k] ? pv[u][k] : first[k] ? z : radd(z, rmul(beta[k], pv[u][k]));
+            }
+            if (any_act) st_row<H>(p + o, pn);
+          }
+        }
+      },
+      [](const BSys &, BState *) {});
 }
 
 // PH_INNER: q = A32 p ; sigma = (p, q) ; alpha = rho / sigma.
 template <int K, class TI>
 __global__ void __launch_bounds__(BT, Occ<K>::spmv_blocks) kb_spmv(const BSys *__restrict__ sys, BState *state,
                                                               BSol *sol, const BCtl *ctl) {
-  __shared__ double sm[32 * 2 * MAXK];
-  if (phase_idle(ctl, PH_INNER)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
+  constexpr int H = Lay<K>::H;
+  __shared__ typename TileSums<K, 1>::Shared sums;
+  __shared__ double sm[8 * 2 * MAXK];
   double *part = ctl->part;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    BState *st = state + T.sys;
-    if (st->phase != PH_INNER) continue;
-    const BSys &S = sys[T.sys];
-    double v[1][K];
+  run_tiles<K, PH_INNER, false, true>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        const TI *__restrict__ p = (const TI *)S.p;
+        TI *__restrict__ q = (TI *)S.q;
+        TileSums<K, 1> acc(sums);
+        tile_spmv<TI, TI, K>(S, T, inner_val<TI>(S), p, [&](int i, size_t o, const double (&aq)[H]) {
+          TI pv[H], qv[H];
+          ld_row_ro<H>(p + o, pv);
 #pragma unroll
-    for (int k = 0; k < K; k++) v[0][k] = 0.0;
-    const TI *__restrict__ p = (const TI *)S.p;
-    TI *__restrict__ q = (TI *)S.q;
-    tile_spmv<TI, TI, K>(S, T, inner_val<TI>(S), p, [&](int r, const double (&aq)[K]) {
-      TI pv[K], qv[K];
-      ld_row<K>(p + (size_t)r * K, pv);
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        qv[k] = (TI)aq[k];
-        v[0][k] = radd(v[0][k], rmul((double)pv[k], (double)qv[k]));
-      }
-      st_row<K>(q + (size_t)r * K, qv);
-    });
-    if (tile_publish<K, 1>(v, part, t, st, S.ntiles, sm)) {
+          for (int k = 0; k < H; k++) {
+            qv[k] = (TI)aq[k];
+            acc.add(i, 0, k, pv[k], qv[k]);
+          }
+          st_row<H>(q + o, qv);
+        });
+        acc.store(T.nrows, j, part, C.idx[j]);
+      },
+      [&](const BSys &S, BState *st) {
       __shared__ double tot[K];
       sys_totals<K>(part, S.tile0, S.ntiles, tot, sm);
       if (threadIdx.x < K) {
@@ -795,84 +918,68 @@ __global__ void __launch_bounds__(BT, Occ<K>::spmv_blocks) kb_spmv(const BSys *_
       }
       __syncthreads();
       if (threadIdx.x == 0) st->ticket = 0;
-    }
-  }
+      });
 }
 
-// PH_INNER: d += alpha p ; r -= alpha q ; z = D r ; (r,z), (r,r) ; inner stop
-// test per rhs ; all rhs stopped -> PH_XUPD.
+// PH_INNER: r -= alpha q ; (r,z), (r,r) with z = D r ; inner stop test per rhs
+// ; all rhs stopped -> PH_XUPD.  (d += alpha p is the next kb_p's or kb_xupd's.)
 template <int K, class TI>
 __global__ void __launch_bounds__(BT, Occ<K>::update_blocks) kb_update(const BSys *__restrict__ sys, BState *state,
                                                                 BSol *sol, const BCtl *ctl) {
-  constexpr int RB = K == 1 ? 4 : 1;
-  __shared__ double sm[32 * 2 * MAXK];
-  if (phase_idle(ctl, PH_INNER)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
+  constexpr int H = Lay<K>::H, L = Lay<K>::L, R = Lay<K>::R;
+  constexpr int RB = K == 1 ? 4 : sizeof(TI) == 8 ? 1 : 2;
+  __shared__ typename TileSums<K, 2>::Shared sums;
+  __shared__ double sm[8 * 2 * MAXK];
   double *part = ctl->part;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    BState *st = state + T.sys;
-    if (st->phase != PH_INNER) continue;
-    const BSys &S = sys[T.sys];
-    TI alpha[K];
-    bool act[K];
+  const int qo = (threadIdx.x % L) * H;
+  run_tiles<K, PH_INNER, true, true>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        TI alpha[H];
+        bool act[H];
+        bool any_act = false;  // a stopped rhs keeps r
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const BSol *so = sol + S.sol0 + k;
-      act[k] = so->active;
-      alpha[k] = (TI)so->alpha;
-    }
-    const TI *__restrict__ p = (const TI *)S.p;
-    const TI *__restrict__ q = (const TI *)S.q;
-    const TI *__restrict__ dinv = (const TI *)S.dinv;
-    TI *__restrict__ d = (TI *)S.d;
-    TI *__restrict__ r32 = (TI *)S.r32;
-    TI *__restrict__ z = (TI *)S.z;
-    double v[2][K];
-#pragma unroll
-    for (int k = 0; k < K; k++) v[0][k] = v[1][k] = 0.0;
-    // a stopped rhs keeps d and r; its z is rewritten as D r, the value it
-    // already holds
-    bool any_act = false;
-#pragma unroll
-    for (int k = 0; k < K; k++) any_act |= act[k];
-    for (int i0 = threadIdx.x; any_act && i0 < T.nrows; i0 += RB * BT) {
-      TI dv[RB][K], pv[RB][K], rv[RB][K], qv[RB][K], dg[RB];
-#pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        const size_t o = ((size_t)T.row0 + i) * K;
-        if (i < T.nrows) {
-          dg[u] = dinv[T.row0 + i];
-          ld_row<K>(d + o, dv[u]);
-          ld_row<K>(p + o, pv[u]);
-          ld_row<K>(r32 + o, rv[u]);
-          ld_row<K>(q + o, qv[u]);
+        for (int k = 0; k < H; k++) {
+          act[k] = C.flags[j][qo + k] & SC_ACTIVE;
+          alpha[k] = (TI)C.alpha[j][qo + k];
+          any_act |= act[k];
         }
-      }
+        const TI *__restrict__ q = (const TI *)S.q;
+        const TI *__restrict__ dinv = (const TI *)S.dinv;
+        TI *__restrict__ r32 = (TI *)S.r32;
+        TileSums<K, 2> acc(sums);
+        for (int i0 = threadIdx.x / L; any_act && i0 < T.nrows; i0 += RB * R) {
+          TI rv[RB][H], qv[RB][H], dg[RB];
 #pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        if (i >= T.nrows) continue;
-        const size_t o = ((size_t)T.row0 + i) * K;
-        TI dn[K], rn[K], zn[K];
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            const size_t o = ((size_t)T.row0 + i) * K + qo;
+            if (i < T.nrows) {
+              dg[u] = dinv[T.row0 + i];
+              ld_row<H>(r32 + o, rv[u]);
+              ld_row<H>(q + o, qv[u]);
+            }
+          }
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-          dn[k] = act[k] ? radd(dv[u][k], rmul(alpha[k], pv[u][k])) : dv[u][k];
-          rn[k] = act[k] ? radd(rv[u][k], -rmul(alpha[k], qv[u][k])) : rv[u][k];
-          zn[k] = rmul(dg[u], rn[k]);
-          if (act[k]) {
-            v[0][k] = radd(v[0][k], rmul((double)rn[k], (double)zn[k]));
-            v[1][k] = radd(v[1][k], rmul((double)rn[k], (double)rn[k]));
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            if (i >= T.nrows) continue;
+            const size_t o = ((size_t)T.row0 + i) * K + qo;
+            TI rn[H];
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+              rn[k] = act[k] ? radd(rv[u][k], -rmul(alpha[k], qv[u][k])) : rv[u][k];
+              if (act[k]) {
+                acc.add(i, 0, k, rn[k], rmul(dg[u], rn[k]));
+                acc.add(i, 1, k, rn[k], rn[k]);
+              }
+            }
+            st_row<H>(r32 + o, rn);
           }
         }
-        st_row<K>(d + o, dn);
-        st_row<K>(r32 + o, rn);
-        st_row<K>(z + o, zn);
-      }
-    }
-    if (tile_publish<K, 2>(v, part, t, st, S.ntiles, sm)) {
+        acc.store(any_act || K > 1 ? T.nrows : 0, j, part, C.idx[j]);
+      },
+      [&](const BSys &S, BState *st) {
       __shared__ double tot[2 * K];
       sys_totals<2 * K>(part, S.tile0, S.ntiles, tot, sm);
       if (threadIdx.x < K) {
@@ -901,67 +1008,67 @@ __global__ void __launch_bounds__(BT, Occ<K>::update_blocks) kb_update(const BSy
         if (!any) move_phase(ctl, st, PH_XUPD);
         st->ticket = 0;
       }
-    }
-  }
+      });
 }
 
-// PH_XUPD: x += scale * d (FP64) for rhs still running ; -> PH_RESID.
+// PH_XUPD: x += scale * (d + alpha p) (FP64; alpha p the step still pending)
+// for rhs still running ; -> PH_RESID.
 template <int K, class TI>
 __global__ void __launch_bounds__(BT, Occ<K>::blocks) kb_xupd(const BSys *__restrict__ sys, BState *state,
                                                               const BSol *sol, const BCtl *ctl) {
-  constexpr int RB = K == 1 ? 4 : 1;
-  if (phase_idle(ctl, PH_XUPD)) return;
-  const BTile *__restrict__ tiles = ctl->tiles;
-  const int ntiles = ctl->ntiles;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BTile T = tiles[t];
-    BState *st = state + T.sys;
-    if (st->phase != PH_XUPD) continue;
-    const BSys &S = sys[T.sys];
-    double sc[K];
+  constexpr int H = Lay<K>::H, L = Lay<K>::L, R = Lay<K>::R;
+  constexpr int RB = 2;
+  const int q = (threadIdx.x % L) * H;
+  run_tiles<K, PH_XUPD, true, true>(
+      sys, state, sol, ctl,
+      [&](const TileChunk<K> &C, int j, const BSys &S, const BTile &T) {
+        double sc[H];
+        TI alpha[H];
+        bool any = false, step = false;
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const BSol *so = sol + S.sol0 + k;
-      sc[k] = so->done == 0 ? so->scale : 0.0;
-    }
-    double *__restrict__ x = S.x;
-    const TI *__restrict__ d = (const TI *)S.d;
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < K; k++) any |= sc[k] != 0.0;
-    for (int i0 = threadIdx.x; any && i0 < T.nrows; i0 += RB * BT) {
-      double xv[RB][K];
-      TI dv[RB][K];
-#pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        const size_t o = ((size_t)T.row0 + i) * K;
-        if (i < T.nrows) {
-          ld_row<K>(x + o, xv[u]);
-          ld_row<K>(d + o, dv[u]);
+        for (int k = 0; k < H; k++) {
+          sc[k] = C.flags[j][q + k] & SC_DONE ? 0.0 : C.beta[j][q + k];
+          alpha[k] = (TI)C.alpha[j][q + k];
+          any |= sc[k] != 0.0;
+          step |= alpha[k] != TI(0);
         }
-      }
+        double *__restrict__ x = S.x;
+        const TI *__restrict__ d = (const TI *)S.d;
+        const TI *__restrict__ p = (const TI *)S.p;
+        for (int i0 = threadIdx.x / L; any && i0 < T.nrows; i0 += RB * R) {
+          double xv[RB][H];
+          TI dv[RB][H], pv[RB][H];
 #pragma unroll
-      for (int u = 0; u < RB; u++) {
-        const int i = i0 + u * BT;
-        if (i >= T.nrows) continue;
-        const size_t o = ((size_t)T.row0 + i) * K;
-        double xn[K];
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            const size_t o = ((size_t)T.row0 + i) * K + q;
+            if (i < T.nrows) {
+              ld_row<H>(x + o, xv[u]);
+              ld_row<H>(d + o, dv[u]);
+              if (step) ld_row<H>(p + o, pv[u]);
+            }
+          }
 #pragma unroll
-        for (int k = 0; k < K; k++) xn[k] = sc[k] != 0.0 ? radd(xv[u][k], rmul(sc[k], (double)dv[u][k])) : xv[u][k];
-        st_row<K>(x + o, xn);
-      }
-    }
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == (unsigned)(S.ntiles - 1);
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-      __threadfence();
-      move_phase(ctl, st, PH_RESID);
-      st->ticket = 0;
-    }
-  }
+          for (int u = 0; u < RB; u++) {
+            const int i = i0 + u * R;
+            if (i >= T.nrows) continue;
+            const size_t o = ((size_t)T.row0 + i) * K + q;
+            double xn[H];
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+              const TI dk = alpha[k] != TI(0) ? radd(dv[u][k], rmul(alpha[k], pv[u][k])) : dv[u][k];
+              xn[k] = sc[k] != 0.0 ? radd(xv[u][k], rmul(sc[k], (double)dk)) : xv[u][k];
+            }
+            st_row<H>(x + o, xn);
+          }
+        }
+      },
+      [&](const BSys &, BState *st) {
+        if (threadIdx.x == 0) {
+          move_phase(ctl, st, PH_RESID);
+          st->ticket = 0;
+        }
+      });
 }
 
 // A slot joins (phase PH_RESID) or leaves (PH_IDLE) between replays: fresh
@@ -985,13 +1092,16 @@ __global__ void kb_dinv(int n, const double *__restrict__ dinv, TI *__restrict__
 // --------------------------------------------------------------- host side
 template <int K, class TI>
 static void capture_iters(Eng *e, cudaStream_t st) {
+  // each kernel's grid is what is resident of it at once
+  const int g = e->sms * Occ<K>::blocks, gr = e->sms * Occ<K>::resid_blocks, gs = e->sms * Occ<K>::spmv_blocks,
+            gu = e->sms * Occ<K>::update_blocks;
   for (int it = 0; it < ITERS; it++) {
-    kb_xupd<K, TI><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
-    kb_resid<K><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
-    kb_init<K, TI><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
-    kb_p<K, TI><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
-    kb_spmv<K, TI><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
-    kb_update<K, TI><<<e->grid, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_xupd<K, TI><<<g, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_resid<K><<<gr, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_init<K, TI><<<g, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_p<K, TI><<<g, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_spmv<K, TI><<<gs, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
+    kb_update<K, TI><<<gu, BT, 0, st>>>(e->d_sys, e->d_state, e->d_sol, e->d_ctl);
   }
 }
 
@@ -1116,7 +1226,7 @@ int psbx_batch_create_prec(void **eng, int max_systems, int max_rows_total, int 
   e->fp64 = inner_bits == 64;
   e->max_sys = max_systems;
   e->max_tiles = max_rows_total / tile_rows(e->K) + max_systems + 1;
-  e->grid = c.sms * 8;
+  e->sms = c.sms;
   e->h_sys.assign(max_systems, BSys());
   e->h_state.assign(max_systems, BState());
   e->used.assign(max_systems, 0);
@@ -1200,9 +1310,9 @@ int psbx_batch_add(void *eng, void *hllMat, const double *d_b, double *d_x, cons
   PsbxCtx &c = psbx_ctx();
   const int K = e->K;
   const size_t n = (size_t)m->rows;
-  // one allocation per slot: r64 (K n doubles), r32 z p q d (5 K n inner values), dinv (n inner values)
+  // one allocation per slot: r64 (K n doubles), r32 p q d (4 K n inner values), dinv (n inner values)
   const size_t ti = e->fp64 ? sizeof(double) : sizeof(float);
-  const size_t bytes = sizeof(double) * K * n + ti * (5 * K + 1) * n + 256;
+  const size_t bytes = sizeof(double) * K * n + ti * (4 * K + 1) * n + 256;
   char *buf = nullptr;
   cudaError_t err = psbx_malloc_async((void **)&buf, bytes, c.stream);
   if (err != cudaSuccess) return psbx_cuda_status(err, "psbx_batch_add");
@@ -1218,11 +1328,10 @@ int psbx_batch_add(void *eng, void *hllMat, const double *d_b, double *d_x, cons
   S.r64 = (double *)buf;
   char *f = buf + sizeof(double) * K * n;
   S.r32 = f;
-  S.z = f + ti * K * n;
-  S.p = f + 2 * ti * K * n;
-  S.q = f + 3 * ti * K * n;
-  S.d = f + 4 * ti * K * n;
-  char *dv = f + 5 * ti * K * n;
+  S.p = f + ti * K * n;
+  S.q = f + 2 * ti * K * n;
+  S.d = f + 3 * ti * K * n;
+  char *dv = f + 4 * ti * K * n;
   S.dinv = dv;
   S.rows = (int)n;
   S.sol0 = s * K;

@@ -22,8 +22,8 @@ import numpy as np
 from . import psb
 
 # device bytes per row and right-hand side the engine needs per request:
-# b, x (FP64), r (FP64), r/z/p/q/d (FP32) and the FP32 inverse diagonal
-BYTES_PER_ROW = 8 + 8 + 8 + 5 * 4 + 4
+# b, x (FP64), r (FP64), r/p/q/d (FP32) and the FP32 inverse diagonal
+BYTES_PER_ROW = 8 + 8 + 8 + 4 * 4 + 4
 
 
 class Pool:
