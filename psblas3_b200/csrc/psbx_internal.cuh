@@ -181,6 +181,21 @@ static inline int psbx_grid_for(long long work, int threads, int perSM = 8) {
   return (int)(need < cap ? need : cap);
 }
 
+// Blocks of a kernel of `threads` threads that are resident at once, at most
+// `most` (a grid for all entries).  The solvers' grid-stride kernels run that
+// many: with 8 per SM for a kernel of which 4 to 6 fit, the rest ran as a
+// second, nearly empty wave.
+template <class F>
+static inline int psbx_resident_grid(F kernel, int threads, int most) {
+  int b = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return most;
+  }
+  const long long g = (long long)b * psbx_ctx().sms;
+  return g > 0 && g < most ? (int)g : most;
+}
+
 // ---------------------------------------------------------------------------
 // Device helpers
 // ---------------------------------------------------------------------------
@@ -341,14 +356,27 @@ __device__ __forceinline__ void final_sum_dd(const double *part, int stride, int
                                              double *smem) {
 #pragma unroll
   for (int k = 0; k < NV; k++) {
-    dd_t a = {0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      dd_t u;
-      u.s = __ldcg(part + 2 * ((size_t)k * stride + i));
-      u.c = __ldcg(part + 2 * ((size_t)k * stride + i) + 1);
-      a = dd_merge(a, u);
+    out[k] = dd_t{0.0, 0.0};
+  }
+  // four blocks' pairs in flight at once: the reads of one block's finaliser
+  // are the tail of every reducing kernel
+  for (int i = threadIdx.x; i < n; i += 4 * blockDim.x) {
+    dd_t u[4][NV];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int j = i + q * (int)blockDim.x;
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const double2 t = j < n ? __ldcg((const double2 *)part + (size_t)k * stride + j) : make_double2(0.0, 0.0);
+        u[q][k] = dd_t{t.x, t.y};
+      }
     }
-    out[k] = a;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (i + q * (int)blockDim.x < n) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) out[k] = dd_merge(out[k], u[q][k]);
+      }
   }
   block_sum_dd<NV>(out, smem);
 }

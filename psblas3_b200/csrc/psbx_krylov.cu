@@ -36,6 +36,57 @@
 #define KLANES 4
 
 // ---------------------------------------------------------------- helpers
+template <class F>
+static int resident_grid(F kernel, int most) { return psbx_resident_grid(kernel, KT, most); }
+
+// The head of a storage row, loaded ahead of its product: for hack size 32
+// the first entry's position and the length, else the row itself.
+struct RowHead {
+  int a, n;
+};
+template <class View> __device__ __forceinline__ RowHead row_head(const View &, int s) { return {s, 0}; }
+template <class View>
+__device__ __forceinline__ double row_dot_head(const View &A, RowHead h, const double *__restrict__ x) {
+  return row_dot(A, h.a, x);
+}
+__device__ __forceinline__ RowHead head32(const HllView &A, int s) {
+  return {ld_ro(A.hkoffs + (s >> 5)) + (s & 31), ld_ro(A.irn + s)};
+}
+__device__ __forceinline__ RowHead row_head(const Hll32View &A, int s) { return head32(A, s); }
+__device__ __forceinline__ RowHead row_head(const Hll32SView &A, int s) { return head32(A, s); }
+__device__ __forceinline__ double row_dot_head(const Hll32View &A, RowHead h, const double *__restrict__ x) {
+  return row_acc<double, double, 8, 32>(A.val + h.a, A.ja + h.a, 32, h.n, x - A.base);
+}
+__device__ __forceinline__ double row_dot_head(const Hll32SView &A, RowHead h, const double *__restrict__ x) {
+  return row_acc_p<double, double, 8, 32>(A.val + h.a, A.ja + h.a, 32, h.n, x - A.base, A.base);
+}
+
+// f(i, m) for the thread's entries of a grid-stride loop, two at a time (m = 1
+// at the end), so that f can issue both entries' loads before it uses them.
+template <class F>
+__device__ __forceinline__ void pairs(int n, F &&f) {
+  const int step = gridDim.x * KT;
+  for (int k = blockIdx.x * KT + threadIdx.x; k < n; k += 2 * step) {
+    const int i[2] = {k, k + step};
+    f(i, k < n - step ? 2 : 1);
+  }
+}
+
+// f(s, row sum) for the thread's rows of a grid-stride loop.
+template <class View, class F>
+__device__ __forceinline__ void each_row_dot(const View &A, const double *__restrict__ x, F &&f) {
+  const int step = gridDim.x * KT;
+  int s = blockIdx.x * KT + threadIdx.x;
+  RowHead h = {0, 0};
+  if (s < A.rows) h = row_head(A, s);
+  for (; s < A.rows; s += step) {
+    RowHead nx = {0, 0};
+    if (s + step < A.rows) nx = row_head(A, s + step);
+    f(s, row_dot_head(A, h, x));
+    h = nx;
+  }
+}
+
 __device__ __forceinline__ bool stopped(const KState *S) { return *((volatile const int *)&S->status) != ST_RUN; }
 
 __device__ __forceinline__ double prec(const double *__restrict__ dinv, int i, double v) {
@@ -181,8 +232,18 @@ __global__ void __launch_bounds__(KT) k_cg_p(KState *S, int n, const double *__r
   if (stopped(S)) return;
   const bool first = S->it == 1;
   const double beta = S->beta;
-  for (int i = blockIdx.x * KT + threadIdx.x; i < n; i += gridDim.x * KT)
-    p[i] = first ? z[i] : radd(z[i], rmul(beta, p[i]));
+  pairs(n, [&](const int (&i)[2], int m) {
+    double zv[2], pv[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) {
+        zv[u] = z[i[u]];
+        if (!first) pv[u] = p[i[u]];
+      }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) p[i[u]] = first ? zv[u] : radd(zv[u], rmul(beta, pv[u]));
+  });
 }
 
 // q = A*p ; sigma = (p,q) ; alpha = rho/sigma
@@ -193,12 +254,11 @@ __global__ void __launch_bounds__(KT) k_cg_spmv(View A, KState *S, const double 
   __shared__ double sm[64];
   if (stopped(S)) return;
   dd_t acc[1] = {{0.0, 0.0}};
-  for (int s = blockIdx.x * KT + threadIdx.x; s < A.rows; s += gridDim.x * KT) {
-    const double t = row_dot(A, s, p);
+  each_row_dot(A, p, [&](int s, double t) {
     const int i = out_row(A, s);
     q[i] = t;
     dd_add_prod(acc[0], ld_ro(p + i), t);
-  }
+  });
   block_sum_dd<1>(acc, sm);
   publish_sums<1>(part, grid, acc);
   if (psbx_last_block(ticket, gridDim.x)) {
@@ -222,30 +282,47 @@ __global__ void __launch_bounds__(KT) k_cg_update(KState *S, int n, const double
                                                   unsigned *__restrict__ ticket, int grid) {
   __shared__ double sm[192];
   if (stopped(S)) return;
+  const bool norms = S->istop == 1;  // the stop test needs max|r| and max|x|
   const double alpha = S->alpha, malpha = -S->alpha;
   dd_t acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
   double mx[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * KT + threadIdx.x; i < n; i += gridDim.x * KT) {
-    const double xi = radd(rmul(alpha, p[i]), x[i]);
-    const double ri = radd(rmul(malpha, q[i]), r[i]);
-    const double zi = prec(dinv, i, ri);
-    x[i] = xi;
-    r[i] = ri;
-    z[i] = zi;
-    dd_add_prod(acc[0], ri, zi);
-    dd_add_prod(acc[1], ri, ri);
-    mx[0] = fmax(mx[0], fabs(ri));
-    mx[1] = fmax(mx[1], fabs(xi));
-  }
+  pairs(n, [&](const int (&i)[2], int m) {
+    double pv[2], qv[2], xv[2], rv[2], dv[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) {
+        pv[u] = p[i[u]];
+        qv[u] = q[i[u]];
+        xv[u] = x[i[u]];
+        rv[u] = r[i[u]];
+        dv[u] = dinv ? ld_ro(dinv + i[u]) : 1.0;  // 1*v is v to the bit
+      }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) {
+        const double xi = radd(rmul(alpha, pv[u]), xv[u]);
+        const double ri = radd(rmul(malpha, qv[u]), rv[u]);
+        const double zi = rmul(dv[u], ri);
+        x[i[u]] = xi;
+        r[i[u]] = ri;
+        z[i[u]] = zi;
+        dd_add_prod(acc[0], ri, zi);
+        dd_add_prod(acc[1], ri, ri);
+        if (norms) {
+          mx[0] = fmax(mx[0], fabs(ri));
+          mx[1] = fmax(mx[1], fabs(xi));
+        }
+      }
+  });
   block_sum_dd<2>(acc, sm);
-  block_max<2>(mx, sm + 128);
+  if (norms) block_max<2>(mx, sm + 128);
   publish_sums<2>(part, grid, acc);
-  publish_max2(part, grid, mx);
+  if (norms) publish_max2(part, grid, mx);
   if (psbx_last_block(ticket, gridDim.x)) {
     dd_t o[2];
-    double m[2];
+    double m[2] = {0.0, 0.0};
     final_sum_dd<2>(part, grid, gridDim.x, o, sm);
-    final_max2(part, grid, gridDim.x, m, sm + 128);
+    if (norms) final_max2(part, grid, gridDim.x, m, sm + 128);
     if (threadIdx.x == 0) {
       if (check_conv(S, dd_value(o[1]), m[0], m[1])) {
         S->status = ST_DONE;
@@ -341,12 +418,11 @@ __global__ void __launch_bounds__(KT) k_bcg_spmv1(View A, KState *S, const doubl
   __shared__ double sm[64];
   if (stopped(S)) return;
   dd_t acc[1] = {{0.0, 0.0}};
-  for (int s = blockIdx.x * KT + threadIdx.x; s < A.rows; s += gridDim.x * KT) {
-    const double t = row_dot(A, s, f);
+  each_row_dot(A, f, [&](int s, double t) {
     const int i = out_row(A, s);
     v[i] = t;
     dd_add_prod(acc[0], ld_ro(q + i), t);
-  }
+  });
   block_sum_dd<1>(acc, sm);
   publish_sums<1>(part, grid, acc);
   if (psbx_last_block(ticket, gridDim.x)) {
@@ -384,13 +460,12 @@ __global__ void __launch_bounds__(KT) k_bcg_spmv2(View A, KState *S, const doubl
   __shared__ double sm[128];
   if (stopped(S)) return;
   dd_t acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (int s = blockIdx.x * KT + threadIdx.x; s < A.rows; s += gridDim.x * KT) {
-    const double ti = row_dot(A, s, z);
+  each_row_dot(A, z, [&](int s, double ti) {
     const int i = out_row(A, s);
     t[i] = ti;
     dd_add_prod(acc[0], ti, ti);
     dd_add_prod(acc[1], ti, ld_ro(sv + i));
-  }
+  });
   block_sum_dd<2>(acc, sm);
   publish_sums<2>(part, grid, acc);
   if (psbx_last_block(ticket, gridDim.x)) {
@@ -421,29 +496,47 @@ __global__ void __launch_bounds__(KT) k_bcg_update(KState *S, int n, const doubl
                                                    int grid) {
   __shared__ double sm[192];
   if (stopped(S)) return;
+  const bool norms = S->istop == 1;  // the stop test needs max|r| and max|x|
   const double alpha = S->alpha, omega = S->omega, momega = -S->omega;
   dd_t acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
   double mx[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * KT + threadIdx.x; i < n; i += gridDim.x * KT) {
-    double xi = radd(rmul(alpha, f[i]), x[i]);
-    xi = radd(rmul(omega, z[i]), xi);
-    const double ri = radd(rmul(momega, t[i]), s[i]);
-    x[i] = xi;
-    r[i] = ri;
-    dd_add_prod(acc[0], ld_ro(q + i), ri);
-    dd_add_prod(acc[1], ri, ri);
-    mx[0] = fmax(mx[0], fabs(ri));
-    mx[1] = fmax(mx[1], fabs(xi));
-  }
+  pairs(n, [&](const int (&i)[2], int m) {
+    double fv[2], zv[2], sv[2], tv[2], qv[2], xv[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) {
+        fv[u] = f[i[u]];
+        xv[u] = x[i[u]];
+        zv[u] = z[i[u]];
+        tv[u] = t[i[u]];
+        sv[u] = s[i[u]];
+        qv[u] = ld_ro(q + i[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (u < m) {
+        double xi = radd(rmul(alpha, fv[u]), xv[u]);
+        xi = radd(rmul(omega, zv[u]), xi);
+        const double ri = radd(rmul(momega, tv[u]), sv[u]);
+        x[i[u]] = xi;
+        r[i[u]] = ri;
+        dd_add_prod(acc[0], qv[u], ri);
+        dd_add_prod(acc[1], ri, ri);
+        if (norms) {
+          mx[0] = fmax(mx[0], fabs(ri));
+          mx[1] = fmax(mx[1], fabs(xi));
+        }
+      }
+  });
   block_sum_dd<2>(acc, sm);
-  block_max<2>(mx, sm + 128);
+  if (norms) block_max<2>(mx, sm + 128);
   publish_sums<2>(part, grid, acc);
-  publish_max2(part, grid, mx);
+  if (norms) publish_max2(part, grid, mx);
   if (psbx_last_block(ticket, gridDim.x)) {
     dd_t o[2];
-    double m[2];
+    double m[2] = {0.0, 0.0};
     final_sum_dd<2>(part, grid, gridDim.x, o, sm);
-    final_max2(part, grid, gridDim.x, m, sm + 128);
+    if (norms) final_max2(part, grid, gridDim.x, m, sm + 128);
     if (threadIdx.x == 0) {
       if (check_conv(S, dd_value(o[1]), m[0], m[1])) {
         S->status = ST_DONE;
@@ -1645,6 +1738,11 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
     psbx_count_launch();
   }
 
+  const int gp = bicg ? resident_grid(k_bcg_p, grid) : resident_grid(k_cg_p, grid);
+  const int gs = resident_grid(k_bcg_s, grid);
+  const int g1 = bicg ? resident_grid(k_bcg_spmv1<View>, grid) : resident_grid(k_cg_spmv<View>, grid);
+  const int g2 = resident_grid(k_bcg_spmv2<View>, grid);
+  const int gu = bicg ? resident_grid(k_bcg_update, grid) : resident_grid(k_cg_update, grid);
   // one captured batch of KGRAPH_ITERS iterations (kept from an earlier call
   // with the same arguments, or captured now)
   cudaGraph_t graph = nullptr;
@@ -1656,18 +1754,18 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
   if (!rc && !gexec) {
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       if (!bicg) {
-        k_cg_p<<<grid, KT, 0, st>>>(S, n, v3, v0);
+        k_cg_p<<<gp, KT, 0, st>>>(S, n, v3, v0);
         psbx_long_rows(A, v0, &S->status, st);
-        k_cg_spmv<View><<<grid, KT, 0, st>>>(A, S, v0, v1, part, ticket, grid);
-        k_cg_update<<<grid, KT, 0, st>>>(S, n, v0, v1, dinv, x, v2, v3, part, ticket, grid);
+        k_cg_spmv<View><<<g1, KT, 0, st>>>(A, S, v0, v1, part, ticket, grid);
+        k_cg_update<<<gu, KT, 0, st>>>(S, n, v0, v1, dinv, x, v2, v3, part, ticket, grid);
       } else {
-        k_bcg_p<<<grid, KT, 0, st>>>(S, n, v1, v3, dinv, v2, v7);
+        k_bcg_p<<<gp, KT, 0, st>>>(S, n, v1, v3, dinv, v2, v7);
         psbx_long_rows(A, v7, &S->status, st);
-        k_bcg_spmv1<View><<<grid, KT, 0, st>>>(A, S, v7, v0, v3, part, ticket, grid);
-        k_bcg_s<<<grid, KT, 0, st>>>(S, n, v1, v3, dinv, v4, v6);
+        k_bcg_spmv1<View><<<g1, KT, 0, st>>>(A, S, v7, v0, v3, part, ticket, grid);
+        k_bcg_s<<<gs, KT, 0, st>>>(S, n, v1, v3, dinv, v4, v6);
         psbx_long_rows(A, v6, &S->status, st);
-        k_bcg_spmv2<View><<<grid, KT, 0, st>>>(A, S, v6, v4, v5, part, ticket, grid);
-        k_bcg_update<<<grid, KT, 0, st>>>(S, n, v7, v6, v4, v5, v0, x, v1, part, ticket, grid);
+        k_bcg_spmv2<View><<<g2, KT, 0, st>>>(A, S, v6, v4, v5, part, ticket, grid);
+        k_bcg_update<<<gu, KT, 0, st>>>(S, n, v7, v6, v4, v5, v0, x, v1, part, ticket, grid);
       }
     }
     e = cudaStreamEndCapture(st, &graph);
@@ -1701,9 +1799,9 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
     if (hS->itx >= opt->itmax) break;
     if ((rc = psbx_long_rows(A, x, nullptr, st))) break;
     if (!bicg)
-      k_cg_init<View><<<grid, KT, 0, st>>>(A, S, b, x, dinv, v2, v3, part, ticket, grid);
+      k_cg_init<View><<<resident_grid(k_cg_init<View>, grid), KT, 0, st>>>(A, S, b, x, dinv, v2, v3, part, ticket, grid);
     else
-      k_bcg_init<View><<<grid, KT, 0, st>>>(A, S, b, x, v1, v0, part, ticket, grid);
+      k_bcg_init<View><<<resident_grid(k_bcg_init<View>, grid), KT, 0, st>>>(A, S, b, x, v1, v0, part, ticket, grid);
     psbx_count_launch(1 + long_launch(A));
     if ((rc = fetch())) break;
     if (hS->status == ST_DONE) break;
@@ -1773,8 +1871,8 @@ static int solve_fcg(const View &A, const double *dinv, const double *b, double 
   if (!rc) {
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       psbx_long_rows(A, v, &S->status, st);
-      k_fcg_spmv<View><<<grid, KT, 0, st>>>(A, S, v, r, q, w, part, ticket, grid);
-      k_fcg_update<<<grid, KT, 0, st>>>(S, n, w, dinv, v, d, q, x, r, part, ticket, grid);
+      k_fcg_spmv<View><<<resident_grid(k_fcg_spmv<View>, grid), KT, 0, st>>>(A, S, v, r, q, w, part, ticket, grid);
+      k_fcg_update<<<resident_grid(k_fcg_update, grid), KT, 0, st>>>(S, n, w, dinv, v, d, q, x, r, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");
@@ -1870,10 +1968,10 @@ static int solve_gmres(const View &A, const double *dinv, const double *b, doubl
     for (int i = 1; i <= nl; i++) {
       k_gm_next<<<grid, KT, 0, st>>>(S, n, i == 1 ? Vk(0) : w, Vk(i - 1), dinv, w1);
       psbx_long_rows(A, w1, &S->status, st);
-      k_gm_spmv<View><<<grid, KT, 0, st>>>(A, S, G, i, w1, Vk(0), w, part, ticket, grid);
+      k_gm_spmv<View><<<resident_grid(k_gm_spmv<View>, grid), KT, 0, st>>>(A, S, G, i, w1, Vk(0), w, part, ticket, grid);
       for (int k = 2; k <= i; k++)
-        k_gm_mgs<<<grid, KT, 0, st>>>(S, G, i, k, n, Vk(k - 2), Vk(k - 1), w, part, ticket, grid);
-      k_gm_norm<<<grid, KT, 0, st>>>(S, G, i, nl, n, Vk(i - 1), w, part, ticket, grid);
+        k_gm_mgs<<<resident_grid(k_gm_mgs, grid), KT, 0, st>>>(S, G, i, k, n, Vk(k - 2), Vk(k - 1), w, part, ticket, grid);
+      k_gm_norm<<<resident_grid(k_gm_norm, grid), KT, 0, st>>>(S, G, i, nl, n, Vk(i - 1), w, part, ticket, grid);
       per_graph += 3 + (i - 1) + long_launch(A);
     }
     k_gm_trsm<<<1, 32, 0, st>>>(S, G);
@@ -1949,10 +2047,10 @@ static int solve_cgs(const View &A, const double *dinv, const double *b, double 
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       k_cgs_p<<<grid, KT, 0, st>>>(S, n, r, q, dinv, uv, p, f);
       psbx_long_rows(A, f, &S->status, st);
-      k_cgs_spmv1<View><<<grid, KT, 0, st>>>(A, S, f, rt, v, part, ticket, grid);
+      k_cgs_spmv1<View><<<resident_grid(k_cgs_spmv1<View>, grid), KT, 0, st>>>(A, S, f, rt, v, part, ticket, grid);
       k_cgs_q<<<grid, KT, 0, st>>>(S, n, uv, v, dinv, q, z, x);
       psbx_long_rows(A, z, &S->status, st);
-      k_cgs_spmv2<View><<<grid, KT, 0, st>>>(A, S, z, rt, x, r, part, ticket, grid);
+      k_cgs_spmv2<View><<<resident_grid(k_cgs_spmv2<View>, grid), KT, 0, st>>>(A, S, z, rt, x, r, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");
@@ -2143,9 +2241,9 @@ static int solve_bicg(const View &A, void *mat, int fmt, const double *dinv, con
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       k_bicg_p<<<grid, KT, 0, st>>>(S, n, z, zt, p, pt);
       psbx_long_rows(A, p, &S->status, st);
-      k_bicg_spmv<View><<<grid, KT, 0, st>>>(A, S, p, pt, q, part, ticket, grid);
+      k_bicg_spmv<View><<<resident_grid(k_bicg_spmv<View>, grid), KT, 0, st>>>(A, S, p, pt, q, part, ticket, grid);
       k_spmv_t<<<grid, KT, 0, st>>>(S, n, tirp, tja, tval, pt, qt);
-      k_bicg_update<<<grid, KT, 0, st>>>(S, n, p, q, qt, dinv, x, r, rt, z, zt, part, ticket, grid);
+      k_bicg_update<<<resident_grid(k_bicg_update, grid), KT, 0, st>>>(S, n, p, q, qt, dinv, x, r, rt, z, zt, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");

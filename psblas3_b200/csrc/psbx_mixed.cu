@@ -23,11 +23,13 @@
 // inner iterations stay close to the FP64 CG's.
 //
 // Per inner iteration, three kernels (as the FP64 CG of psbx_krylov.cu):
-//   p = z + beta p (z = d .* rh formed on the fly)
+//   xh = alpha p + xh with the last iteration's alpha and p (p is read here
+//     anyway, so the update need not read it), p = z + beta p (z = d .* rh
+//     formed on the fly)
 //   q = A p (FP32 product, two rows per thread: exact FP64 products added
 //     in FP64, rounded once) and sigma = (p, q), alpha = rho / sigma
-//   xh = alpha p + xh, rh = -alpha q + rh, z = d .* rh, rho' = (rh, z),
-//     ||rh||^2, and the replacement test
+//   rh = -alpha q + rh, z = d .* rh, rho' = (rh, z), ||rh||^2, and the
+//     replacement test
 // Every kernel returns at once when the status word is not RUN, so eight
 // iterations are one CUDA graph replayed until the host sees a replacement
 // request (then the replacement graph runs: fold, FP64 residual) or the end.
@@ -88,16 +90,21 @@ __device__ __forceinline__ void pair32(const HllViewF &A, int off, int n0, int n
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      if (j + u < n0) a0 = radd(a0, rmul((double)v[u].x, (double)x0[u]));
-      if (j + u < n1) a1 = radd(a1, rmul((double)v[u].y, (double)x1[u]));
+      // (exact products: one fused multiply-add rounds as the two do)
+      if (j + u < n0) a0 = __fma_rn((double)v[u].x, (double)x0[u], a0);
+      if (j + u < n1) a1 = __fma_rn((double)v[u].y, (double)x1[u], a1);
     }
   }
   y0 = (float)a0;
   y1 = (float)a1;
 }
 
+// (the product of two floats is exact in FP64: its error term is zero)
 __device__ __forceinline__ void exact_add(dd_t &acc, float a, float b) {
-  dd_add_prod(acc, (double)a, (double)b);
+  double s, t;
+  two_sum(acc.s, rmul((double)a, (double)b), s, t);
+  acc.s = s;
+  acc.c = radd(acc.c, t);
 }
 
 template <int NS>
@@ -134,10 +141,18 @@ __global__ void __launch_bounds__(MT) k_mx_setup(int n, const double *__restrict
   }
 }
 
-// x = x + xh (FP64) ; xh = 0
-__global__ void __launch_bounds__(MT) k_mx_fold(int n, double *__restrict__ x, float *__restrict__ xh) {
+// The step alpha p that xh has not taken yet (alpha 0: none is pending).
+__device__ __forceinline__ float step_el(float alpha, float p, float xh) {
+  return alpha != 0.0f ? raddf(rmulf(alpha, p), xh) : xh;
+}
+
+// x = x + xh (FP64), xh with its last step ; xh = 0.  (The replacement that
+// follows clears alpha.)
+__global__ void __launch_bounds__(MT) k_mx_fold(const MState *S, int n, const float *__restrict__ p,
+                                                double *__restrict__ x, float *__restrict__ xh) {
+  const float alpha = (float)S->alpha;
   for (int i = blockIdx.x * MT + threadIdx.x; i < n; i += gridDim.x * MT) {
-    x[i] = radd(x[i], (double)xh[i]);
+    x[i] = radd(x[i], (double)step_el(alpha, p[i], xh[i]));
     xh[i] = 0.0f;
   }
 }
@@ -171,6 +186,7 @@ __global__ void __launch_bounds__(MT) k_mx_resid(View A, MState *S, const double
       const double rhonew = dd_value(o[0]);
       const double rt = sqrt(dd_value(o[1]));
       const bool broke = S->status == MX_BREAK;
+      S->alpha = 0.0;  // folded into x
       S->rtrue = rt;
       S->refreshes += 1;
       const bool conv = S->bn2 == 0.0 ? rt <= S->eps : rt <= S->eps * S->bn2;
@@ -199,25 +215,33 @@ __global__ void __launch_bounds__(MT) k_mx_resid(View A, MState *S, const double
 // first threads one at a time).
 __device__ __forceinline__ float4 ld4(const float *p, int k) { return ld_stream((const float4 *)p + k); }
 
-// p = z (after a restart) or p = z + beta p, z = d .* rh
-__device__ __forceinline__ float p_el(bool first, float beta, float d, float r, float p) {
+// xh = alpha p + xh, the last step ; p = z (after a restart) or p = z + beta p,
+// z = d .* rh
+__device__ __forceinline__ float p_el(bool first, float beta, float alpha, float d, float r, float p, float &xh) {
   const float z = rmulf(d, r);
+  xh = step_el(alpha, p, xh);
   return first ? z : raddf(z, rmulf(beta, p));
 }
 __global__ void __launch_bounds__(MT) k_mx_p(MState *S, int n, const float *__restrict__ d32,
-                                             const float *__restrict__ rh, float *__restrict__ p) {
+                                             const float *__restrict__ rh, float *__restrict__ p,
+                                             float *__restrict__ xh) {
   if (mx_stopped(S)) return;
   const bool first = S->first != 0;
-  const float beta = (float)S->beta;
+  const float beta = (float)S->beta, alpha = (float)S->alpha;
   const int n4 = n >> 2;
   for (int k = blockIdx.x * MT + threadIdx.x; k < n4; k += gridDim.x * MT) {
     const float4 d = ld4(d32, k), r = ld4(rh, k), q = ((const float4 *)p)[k];
-    ((float4 *)p)[k] = make_float4(p_el(first, beta, d.x, r.x, q.x), p_el(first, beta, d.y, r.y, q.y),
-                                   p_el(first, beta, d.z, r.z, q.z), p_el(first, beta, d.w, r.w, q.w));
+    float4 x = ((const float4 *)xh)[k];
+    ((float4 *)p)[k] =
+        make_float4(p_el(first, beta, alpha, d.x, r.x, q.x, x.x), p_el(first, beta, alpha, d.y, r.y, q.y, x.y),
+                    p_el(first, beta, alpha, d.z, r.z, q.z, x.z), p_el(first, beta, alpha, d.w, r.w, q.w, x.w));
+    ((float4 *)xh)[k] = x;
   }
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
     const int i = 4 * n4 + threadIdx.x;
-    p[i] = p_el(first, beta, d32[i], rh[i], p[i]);
+    float x = xh[i];
+    p[i] = p_el(first, beta, alpha, d32[i], rh[i], p[i], x);
+    xh[i] = x;
   }
 }
 
@@ -284,48 +308,46 @@ __global__ void __launch_bounds__(MT, 4) k_mx_spmv(HllViewF A, MState *S, const 
     if (threadIdx.x == 0) {
       const double sigma = dd_value(o[0]);
       S->first = 0;
-      if (sigma == 0.0) S->status = MX_BREAK;
-      else S->alpha = S->rho / sigma;
+      if (sigma == 0.0) {
+        S->status = MX_BREAK;
+        S->alpha = 0.0;  // no step (the last one is in xh since k_mx_p)
+      } else {
+        S->alpha = S->rho / sigma;
+      }
       *ticket = 0;
     }
   }
 }
 
-// xh = alpha p + xh ; rh = -alpha q + rh ; rho' = (rh, d.*rh) ; ||rh||^2 ;
-// replacement test
-__device__ __forceinline__ void upd_el(float af, float maf, float p, float q, float d, float &xh, float &r,
-                                       dd_t (&acc)[2]) {
-  xh = raddf(rmulf(af, p), xh);
+// rh = -alpha q + rh ; rho' = (rh, d.*rh) ; ||rh||^2 ; replacement test
+__device__ __forceinline__ void upd_el(float maf, float q, float d, float &r, dd_t (&acc)[2]) {
   r = raddf(rmulf(maf, q), r);
   const float z = rmulf(d, r);
   exact_add(acc[0], r, z);
   exact_add(acc[1], r, r);
 }
-__global__ void __launch_bounds__(MT) k_mx_update(MState *S, int n, const float *__restrict__ p,
-                                                  const float *__restrict__ q, const float *__restrict__ d32,
-                                                  float *__restrict__ xh, float *__restrict__ rh,
+__global__ void __launch_bounds__(MT) k_mx_update(MState *S, int n, const float *__restrict__ q,
+                                                  const float *__restrict__ d32, float *__restrict__ rh,
                                                   double *__restrict__ part, unsigned *__restrict__ ticket,
                                                   int grid) {
   __shared__ double sm[128];
   if (mx_stopped(S)) return;
-  const float af = (float)S->alpha, maf = -af;
+  const float maf = -(float)S->alpha;
   dd_t acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
   const int n4 = n >> 2;
   for (int k = blockIdx.x * MT + threadIdx.x; k < n4; k += gridDim.x * MT) {
-    const float4 pp = ld4(p, k), qq = ld4(q, k), d = ld4(d32, k);
-    float4 x = ((const float4 *)xh)[k], r = ((const float4 *)rh)[k];
-    upd_el(af, maf, pp.x, qq.x, d.x, x.x, r.x, acc);
-    upd_el(af, maf, pp.y, qq.y, d.y, x.y, r.y, acc);
-    upd_el(af, maf, pp.z, qq.z, d.z, x.z, r.z, acc);
-    upd_el(af, maf, pp.w, qq.w, d.w, x.w, r.w, acc);
-    ((float4 *)xh)[k] = x;
+    const float4 qq = ld4(q, k), d = ld4(d32, k);
+    float4 r = ((const float4 *)rh)[k];
+    upd_el(maf, qq.x, d.x, r.x, acc);
+    upd_el(maf, qq.y, d.y, r.y, acc);
+    upd_el(maf, qq.z, d.z, r.z, acc);
+    upd_el(maf, qq.w, d.w, r.w, acc);
     ((float4 *)rh)[k] = r;
   }
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
     const int i = 4 * n4 + threadIdx.x;
-    float x = xh[i], r = rh[i];
-    upd_el(af, maf, p[i], q[i], d32[i], x, r, acc);
-    xh[i] = x;
+    float r = rh[i];
+    upd_el(maf, q[i], d32[i], r, acc);
     rh[i] = r;
   }
   block_sum_dd<2>(acc, sm);
@@ -401,18 +423,21 @@ static int mx_solve(const View &A64, const HllViewF &A32, bool shortRows, const 
   int gq = (n / 4 + MT - 1) / MT, gs = ((n + 1) / 2 + MT - 1) / MT;
   gq = gq < 1 ? 1 : (gq > grid ? grid : gq);
   gs = gs < 1 ? 1 : (gs > grid ? grid : gs);
+  const int gp = psbx_resident_grid(k_mx_p, MT, gq), gu = psbx_resident_grid(k_mx_update, MT, gq),
+            gres = psbx_resident_grid(k_mx_resid<View>, MT, grid);
+  gs = shortRows ? psbx_resident_grid(k_mx_spmv<8>, MT, gs) : psbx_resident_grid(k_mx_spmv<4>, MT, gs);
   rc = capture(&gi, &ei, [&]() {
     for (int k = 0; k < MX_ITERS; k++) {
-      k_mx_p<<<gq, MT, 0, st>>>(S, n, d32, rh, p);
+      k_mx_p<<<gp, MT, 0, st>>>(S, n, d32, rh, p, xh);
       if (shortRows) k_mx_spmv<8><<<gs, MT, 0, st>>>(A32, S, p, q, part, ticket, gs);
       else k_mx_spmv<4><<<gs, MT, 0, st>>>(A32, S, p, q, part, ticket, gs);
-      k_mx_update<<<gq, MT, 0, st>>>(S, n, p, q, d32, xh, rh, part, ticket, gq);
+      k_mx_update<<<gu, MT, 0, st>>>(S, n, q, d32, rh, part, ticket, gu);
     }
   });
   if (!rc) rc = capture(&gr, &er, [&]() {
-    k_mx_fold<<<grid, MT, 0, st>>>(n, x, xh);
+    k_mx_fold<<<grid, MT, 0, st>>>(S, n, p, x, xh);
     psbx_long_rows(A64, x, nullptr, st);
-    k_mx_resid<View><<<grid, MT, 0, st>>>(A64, S, b, x, d32, rh, part, ticket, grid);
+    k_mx_resid<View><<<gres, MT, 0, st>>>(A64, S, b, x, d32, rh, part, ticket, gres);
   });
   auto fetch = [&]() -> int {
     PSBX_CK(cudaMemcpyAsync(hS, S, sizeof(MState), cudaMemcpyDeviceToHost, st));
