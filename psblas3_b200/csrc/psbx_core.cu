@@ -40,8 +40,7 @@ static int ctx_create(int dev) {
   PSBX_CK(cudaMalloc(&c.d_part, sizeof(double) * 2 * PSBX_NLANES * PSBX_MAX_PART));
   PSBX_CK(cudaMalloc(&c.d_ticket, sizeof(unsigned) * 64));
   PSBX_CK(cudaMemset(c.d_ticket, 0, sizeof(unsigned) * 64));
-  PSBX_CK(cudaMalloc(&c.d_res, sizeof(double) * 64));
-  PSBX_CK(cudaHostAlloc(&c.h_res, sizeof(double) * 64, cudaHostAllocDefault));
+  PSBX_CK(cudaHostAlloc(&c.h_res, sizeof(double) * 64, cudaHostAllocMapped));
   cudaMemPoolProps pp;
   memset(&pp, 0, sizeof(pp));
   pp.allocType = cudaMemAllocationTypePinned;
@@ -81,7 +80,6 @@ static void ctx_destroy() {
   cudaStreamSynchronize(c.stream);
   cudaFree(c.d_part);
   cudaFree(c.d_ticket);
-  cudaFree(c.d_res);
   cudaFreeHost(c.h_res);
   cudaStreamSynchronize(c.defaultStream);
   for (cudaEvent_t e : c.xev) cudaEventDestroy(e);

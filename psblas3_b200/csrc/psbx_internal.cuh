@@ -135,8 +135,7 @@ struct PsbxCtx {
   cudaDeviceProp prop;
   double *d_part = nullptr;       // [PSBX_NLANES][PSBX_MAX_PART]
   unsigned *d_ticket = nullptr;   // [64] zero-initialised, reset by users
-  double *d_res = nullptr;        // [64] reduction results
-  double *h_res = nullptr;        // pinned [64]
+  double *h_res = nullptr;        // pinned [64]: reduction results, written by the kernels
   // Stream-ordered workspace of the solvers comes from this pool, which
   // keeps up to PSBX_POOL_KEEP bytes of freed memory mapped between calls:
   // with nothing kept, every solve remapped its workspace (1 GB for CG on
