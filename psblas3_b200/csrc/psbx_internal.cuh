@@ -490,6 +490,7 @@ struct Hll32WView : HllView {};
 // operators): a row's entries are read as one predicated group, so all of its
 // index and value loads are in flight at once instead of one after another.
 struct Hll32SView : HllView {};
+struct EllSView : EllView {};  // the same for ELL
 #define PSBX_SHORT_ROW 16
 
 // Unrolled in-order accumulation over one row whose j-th entry sits at
@@ -520,10 +521,24 @@ __device__ __forceinline__ double row_acc(const VT *__restrict__ vp, const int *
 #pragma unroll
     for (int u = 0; u < U; u++) acc = radd(acc, rmul((double)v[u], (double)xv[u]));
   }
-  for (; j < n; j++) {
-    const int c = ld_stream(jp + j * st);
-    const VT v = ld_stream(vp + j * st);
-    acc = radd(acc, rmul((double)v, (double)ld_ro(xb + c)));
+  // the tail in predicated groups of TU: one entry at a time it was a chain of
+  // up to U - 1 more pairs of round trips, as long again as a 27-entry row
+  constexpr int TU = U < 4 ? U : 4;
+  for (; j < n; j += TU) {
+    int c[TU];
+    VT v[TU];
+#pragma unroll
+    for (int u = 0; u < TU; u++) {
+      const bool ok = j + u < n;
+      c[u] = ok ? ld_stream(jp + (j + u) * st) : 0;
+      v[u] = ok ? ld_stream(vp + (j + u) * st) : VT(0);
+    }
+    XT xv[TU];
+#pragma unroll
+    for (int u = 0; u < TU; u++) xv[u] = j + u < n ? ld_ro(xb + c[u]) : XT(0);
+#pragma unroll
+    for (int u = 0; u < TU; u++)
+      if (j + u < n) acc = radd(acc, rmul((double)v[u], (double)xv[u]));
   }
   return acc;
 }
@@ -570,6 +585,49 @@ __device__ __forceinline__ double row_acc_p(const VT *__restrict__ vp, const int
   return acc;
 }
 
+// FP32 products of the row pair (s0, s0 + 1), s0 even, of a hack-32 matrix,
+// both in one thread.  The two rows are adjacent in every column of their
+// hack, so entry j of both is one float2 (values) and one int2 (indices):
+// each load instruction of a warp moves 256 bytes, as the FP64 kernels' do,
+// where one row per thread would move 128 (measured: 3.6 TB/s for one row
+// per thread on the 7-point operator, against 6.25 TB/s for FP64).  Each
+// row still adds its own entries in stored order, in FP64, from exact
+// products, and rounds once.  Slots past a row's length (padding of the
+// hack) may be loaded but are never added.
+template <int U>
+__device__ __forceinline__ void pair32(const HllViewF &A, int off, int n0, int n1, const float *__restrict__ x,
+                                       float &y0, float &y1) {
+  const float *vp = A.val + off;
+  const int *jp = A.ja + off;
+  const float *xb = x - A.base;
+  const int n = max(n0, n1);
+  double a0 = 0.0, a1 = 0.0;
+  for (int j = 0; j < n; j += U) {
+    int2 c[U];
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const bool ok = j + u < n;
+      c[u] = ok ? ld_stream((const int2 *)(jp + (j + u) * 32)) : make_int2(A.base, A.base);
+      v[u] = ok ? ld_stream((const float2 *)(vp + (j + u) * 32)) : make_float2(0.0f, 0.0f);
+    }
+    float x0[U], x1[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      x0[u] = j + u < n0 ? ld_ro(xb + c[u].x) : 0.0f;
+      x1[u] = j + u < n1 ? ld_ro(xb + c[u].y) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      // (exact products: one fused multiply-add rounds as the two do)
+      if (j + u < n0) a0 = __fma_rn((double)v[u].x, (double)x0[u], a0);
+      if (j + u < n1) a1 = __fma_rn((double)v[u].y, (double)x1[u], a1);
+    }
+  }
+  y0 = (float)a0;
+  y1 = (float)a1;
+}
+
 __device__ __forceinline__ double row_dot(const Hll32SView &A, int s, const double *__restrict__ x) {
   const int off = ld_ro(A.hkoffs + (s >> 5)) + (s & 31);
   return row_acc_p<double, double, 8, 32>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base, A.base);
@@ -607,6 +665,10 @@ __device__ __forceinline__ double row_dot(const HllViewF &A, int s, const float 
 
 __device__ __forceinline__ double row_dot(const EllView &A, int r, const double *__restrict__ x) {
   return row_acc<double, double, 8, 0>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base);
+}
+
+__device__ __forceinline__ double row_dot(const EllSView &A, int r, const double *__restrict__ x) {
+  return row_acc_p<double, double, 8, 0>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base, A.base);
 }
 
 __device__ __forceinline__ double row_dot(const EllViewF &A, int r, const float *__restrict__ x) {
@@ -653,6 +715,7 @@ __device__ __forceinline__ int out_row(const Hll32WView &A, int s) { return A.pe
 __device__ __forceinline__ int out_row(const Hll32SView &A, int s) { return A.perm ? ld_ro(A.perm + s) : s; }
 __device__ __forceinline__ int out_row(const HllViewF &A, int s) { return A.perm ? ld_ro(A.perm + s) : s; }
 __device__ __forceinline__ int out_row(const EllView &, int r) { return r; }
+__device__ __forceinline__ int out_row(const EllSView &, int r) { return r; }
 __device__ __forceinline__ int out_row(const EllViewF &, int r) { return r; }
 __device__ __forceinline__ int out_row(const CsrView &, int r) { return r; }
 
@@ -679,6 +742,11 @@ static inline Hll32WView hll32w_view(const HllView &v) {
 static inline Hll32SView hll32s_view(const HllView &v) {
   Hll32SView w;
   static_cast<HllView &>(w) = v;
+  return w;
+}
+static inline EllSView ells_view(const EllView &v) {
+  EllSView w;
+  static_cast<EllView &>(w) = v;
   return w;
 }
 // A hack-32 matrix with no wide hacks whose rows all hold at most

@@ -56,49 +56,6 @@ __device__ __forceinline__ bool mx_stopped(const MState *S) {
   return *((volatile const int *)&S->status) != MX_RUN;
 }
 
-// FP32 products of the row pair (s0, s0 + 1), s0 even, of a hack-32 matrix,
-// both in one thread.  The two rows are adjacent in every column of their
-// hack, so entry j of both is one float2 (values) and one int2 (indices):
-// each load instruction of a warp moves 256 bytes, as the FP64 kernels' do,
-// where one row per thread would move 128 (measured: 3.6 TB/s for one row
-// per thread on the 7-point operator, against 6.25 TB/s for FP64).  Each
-// row still adds its own entries in stored order, in FP64, from exact
-// products, and rounds once.  Slots past a row's length (padding of the
-// hack) may be loaded but are never added.
-template <int U>
-__device__ __forceinline__ void pair32(const HllViewF &A, int off, int n0, int n1, const float *__restrict__ x,
-                                       float &y0, float &y1) {
-  const float *vp = A.val + off;
-  const int *jp = A.ja + off;
-  const float *xb = x - A.base;
-  const int n = max(n0, n1);
-  double a0 = 0.0, a1 = 0.0;
-  for (int j = 0; j < n; j += U) {
-    int2 c[U];
-    float2 v[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const bool ok = j + u < n;
-      c[u] = ok ? ld_stream((const int2 *)(jp + (j + u) * 32)) : make_int2(A.base, A.base);
-      v[u] = ok ? ld_stream((const float2 *)(vp + (j + u) * 32)) : make_float2(0.0f, 0.0f);
-    }
-    float x0[U], x1[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      x0[u] = j + u < n0 ? ld_ro(xb + c[u].x) : 0.0f;
-      x1[u] = j + u < n1 ? ld_ro(xb + c[u].y) : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      // (exact products: one fused multiply-add rounds as the two do)
-      if (j + u < n0) a0 = __fma_rn((double)v[u].x, (double)x0[u], a0);
-      if (j + u < n1) a1 = __fma_rn((double)v[u].y, (double)x1[u], a1);
-    }
-  }
-  y0 = (float)a0;
-  y1 = (float)a1;
-}
-
 // (the product of two floats is exact in FP64: its error term is zero)
 __device__ __forceinline__ void exact_add(dd_t &acc, float a, float b) {
   double s, t;

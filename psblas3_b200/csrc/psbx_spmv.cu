@@ -372,8 +372,16 @@ CsrView csr_view(const CsrDevice *m) {
 
 // --------------------------------------------------------------- row kernels
 // MODE 0: y = alpha*acc + beta*y ; MODE 1: beta == 0, y not read.
+// Blocks of SPMV_T per SM that a kernel's registers allow, the fastest of 4, 5,
+// 6 and 8 for each: without a bound the compiler keeps to 32 registers (8
+// blocks) and a group of 8 entries waits in pieces.  27-point HLL 200^3 428 us
+// at 8, 407 at 5 (6.69 TB/s), 410 at 6; 100^3 58 and 51; ELL 101^3 67.6 and
+// 56.2 at 4; 7-point 100^3 HLL 16.4 at 5, 15.3 at 6; ELL 20.5 at 6, 18.5 at 5.
+template <class View> constexpr int spmv_blocks = 5;
+template <> constexpr int spmv_blocks<Hll32SView> = 6;
+template <> constexpr int spmv_blocks<EllView> = 4;
 template <class View, int MODE>
-__global__ void __launch_bounds__(SPMV_T) k_spmv_rows(View A, double alpha, const double *__restrict__ x,
+__global__ void __launch_bounds__(SPMV_T, spmv_blocks<View>) k_spmv_rows(View A, double alpha, const double *__restrict__ x,
                                                       double beta, double *__restrict__ y) {
   const int s = blockIdx.x * SPMV_T + threadIdx.x;
   if (s >= A.rows) return;
@@ -384,7 +392,7 @@ __global__ void __launch_bounds__(SPMV_T) k_spmv_rows(View A, double alpha, cons
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(SPMV_T) k_hll_spmv_f32(HllViewF A, float alpha, const float *__restrict__ x,
+__global__ void __launch_bounds__(SPMV_T, 6) k_hll_spmv_f32(HllViewF A, float alpha, const float *__restrict__ x,
                                                          float beta, float *__restrict__ y) {
   const int s = blockIdx.x * SPMV_T + threadIdx.x;
   if (s >= A.rows) return;
@@ -805,9 +813,34 @@ extern "C" int psbx_hll_spmv_host(void *deviceMat, double alpha, const double *x
   return SPGPU_SUCCESS;
 }
 
+// FP32, hack size 32, short rows: two adjacent rows per thread (entry j of both
+// is one float2 and one int2, 256 bytes per warp load where one row moves
+// 128), the sums of k_hll_spmv_f32 bit for bit.  7-point 100^3: 16.4 us, one
+// row per thread 20.5; the 27-point rows are the other way round (64 us
+// against 39): a pair holds more loads in flight than the registers take.
+template <int MODE>
+__global__ void __launch_bounds__(SPMV_T, 5) k_hll_spmv_f32_pairs(HllViewF A, float alpha, const float *__restrict__ x,
+                                                               float beta, float *__restrict__ y) {
+  const int s0 = 2 * (blockIdx.x * SPMV_T + threadIdx.x);
+  if (s0 >= A.rows) return;
+  const bool two = s0 + 1 < A.rows;
+  const int off = ld_ro(A.hkoffs + (s0 >> 5)) + (s0 & 31);
+  const int n0 = ld_ro(A.irn + s0), n1 = two ? ld_ro(A.irn + s0 + 1) : 0;
+  const int d0 = out_row(A, s0), d1 = two ? out_row(A, s0 + 1) : 0;
+  float a0, a1;
+  pair32<8>(A, off, n0, n1, x, a0, a1);
+  const float t0 = rmulf(alpha, a0);
+  y[d0] = MODE == 1 ? t0 : raddf(t0, rmulf(beta, y[d0]));
+  if (two) {
+    const float t1 = rmulf(alpha, a1);
+    y[d1] = MODE == 1 ? t1 : raddf(t1, rmulf(beta, y[d1]));
+  }
+}
+
 int psbx_launch_ell_spmv(const EllDevice *m, double alpha, const double *x, double beta, double *y,
                          cudaStream_t st) {
   if (m->dataType != SPGPU_TYPE_DOUBLE) return SPGPU_UNSUPPORTED;
+  if (m->maxRowSize <= PSBX_SHORT_ROW) return launch_rows(ells_view(ell_view(m)), alpha, x, beta, y, st);
   return launch_rows(ell_view(m), alpha, x, beta, y, st);
 }
 
@@ -834,6 +867,15 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
     PSBX_LAUNCH_CK("k_f32_scale");
     return SPGPU_SUCCESS;
   }
+  if (m->hackSize == 32 && m->maxRowLen >= 0 && m->maxRowLen <= PSBX_SHORT_ROW) {
+    const int gp = ((A.rows + 1) / 2 + SPMV_T - 1) / SPMV_T;
+    if (beta == 0.0f)
+      k_hll_spmv_f32_pairs<1><<<gp, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    else
+      k_hll_spmv_f32_pairs<0><<<gp, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    PSBX_LAUNCH_CK("k_hll_spmv_f32_pairs");
+    return SPGPU_SUCCESS;
+  }
   const int g = (A.rows + SPMV_T - 1) / SPMV_T;
   if (beta == 0.0f)
     k_hll_spmv_f32<1><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
@@ -848,7 +890,7 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
 // is exact in FP64, the products are added in FP64 in stored order and the
 // sum is rounded to FP32 once -- then y = alpha*sum + beta*y in FP32.
 template <int MODE>
-__global__ void __launch_bounds__(SPMV_T) k_ell_spmv_f32(EllViewF A, float alpha, const float *__restrict__ x,
+__global__ void __launch_bounds__(SPMV_T, 6) k_ell_spmv_f32(EllViewF A, float alpha, const float *__restrict__ x,
                                                          float beta, float *__restrict__ y) {
   const int r = blockIdx.x * SPMV_T + threadIdx.x;
   if (r >= A.rows) return;
