@@ -1,0 +1,58 @@
+"""Row kernels at the edges of their forms: row lengths 0 .. 16 (short-row
+HLL and ELL, FP32 row pairs) and 0 .. 35 (groups of 8 entries, tails of 1 to 7
+in groups of 4), odd row counts, a row permutation, alpha and beta; FP64
+products bit for bit the CPU csmv's, FP32 ones the FP64 row sum rounded once."""
+import numpy as np
+import pytest
+
+import oracle as O
+from psblas3_b200 import gen
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, longest, seed):
+    rng = np.random.default_rng(seed)
+    k = np.minimum(rng.integers(0, longest + 1, n), n)
+    k[-1] = min(longest, n)  # the longest row there is
+    irp = np.concatenate([[1], 1 + np.cumsum(k)]).astype(np.int32)
+    ja = np.concatenate([np.sort(rng.choice(n, size=c, replace=False)) + 1 for c in k]).astype(np.int32)
+    return irp, ja, rng.standard_normal(len(ja))
+
+
+def _hll(psb, irp, ja, va, perm=None):
+    import torch
+    n = len(irp) - 1
+    d = [torch.from_numpy(a).cuda() for a in (irp, ja, va)]
+    p = None if perm is None else torch.from_numpy(perm).cuda()
+    torch.cuda.synchronize()
+    return psb.HllMat.from_csr_device(n, n, len(ja), *(t.data_ptr() for t in d), 32, None if p is None else p.data_ptr())
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1001])
+@pytest.mark.parametrize("longest", [16, 17, 35])
+@pytest.mark.parametrize("alpha,beta", [(1.0, 0.0), (-0.5, 2.0)])
+def test_row_forms(psb, n, longest, alpha, beta):
+    irp, ja, va = _rows(n, longest, n + longest)
+    rng = np.random.default_rng(1)
+    x, y0 = rng.uniform(-1, 1, (2, n))
+    ref = O.csr_csmv(irp, ja, va, alpha, x, beta, y0.copy())
+    ia, _, _ = gen.csr_to_coo(irp, ja, va)
+    perm = rng.permutation(n).astype(np.int32)
+    mats = [_hll(psb, irp, ja, va), _hll(psb, irp, ja, va, perm), psb.EllMat.from_coo_gpu(n, ia, ja, va)]
+    for A in mats:
+        X, Y = psb.DVect.bld(x), psb.DVect.bld(y0)
+        psb.psb_spmm(alpha, A, X, beta, Y)
+        assert np.array_equal(Y.get_vect(), ref)
+    # FP32: exact products added in FP64 in stored order, rounded once, then
+    # alpha * sum + beta * y in FP32
+    v32, x32, y32 = va.astype(np.float32), x.astype(np.float32), y0.astype(np.float32)
+    s = O.csr_csmv(irp, ja, v32.astype(np.float64), 1.0, x32.astype(np.float64), 0.0, np.zeros(n)).astype(np.float32)
+    ref32 = np.float32(alpha) * s
+    if beta != 0.0:
+        ref32 = ref32 + np.float32(beta) * y32
+    for A in mats[:2]:
+        A.make_single()
+        X, Y = psb.DVect.bld(x32), psb.DVect.bld(y32)
+        A.spmv(alpha, X, beta, Y)
+        assert np.array_equal(Y.get_vect(), ref32)
