@@ -442,9 +442,12 @@ int psbx_DefaultSolverOptions(psbx_SolverOptions *opt);
  *   b, x  MultiVectDevice (x holds x0 on entry, the solution on exit)
  * Scalars stay on the device; the stop test runs every iteration on the
  * device; the host reads a status word once per captured batch of
- * iterations.  Returns 0 (converged or itmax reached, as the reference),
- * or an error code; opt->iter and opt->err are filled like psb_krylov's
- * iter and err. */
+ * iterations -- or once per solve: CG and BiCGSTAB of systems whose vectors
+ * fit the SMs' shared memory (about 700,000 / 510,000 rows, no wide hacks,
+ * itmax <= 100000) run as one cooperative kernel.  Returns 0 (converged or
+ * itmax reached, as the reference), or an error code (PSBX_TIMEOUT: a wait
+ * between that kernel's blocks ran past its bound); opt->iter and opt->err
+ * are filled like psb_krylov's iter and err. */
 int psbx_dkrylov(const char *method, void *mat, int fmt, void *dinv,
                  void *b, void *x, psbx_SolverOptions *opt);
 
