@@ -378,7 +378,9 @@ CsrView csr_view(const CsrDevice *m) {
 // at 8, 407 at 5 (6.69 TB/s), 410 at 6; 100^3 58 and 51; ELL 101^3 67.6 and
 // 56.2 at 4; 7-point 100^3 HLL 16.4 at 5, 15.3 at 6; ELL 20.5 at 6, 18.5 at 5.
 // The FP32 rows need half the bytes in flight per load: 27-point 100^3 43.1 at
-// 5, 39.3 at 6, 37.0 at 8 (with the grouped tail; 41.6 without).
+// 5, 39.3 at 6, 37.0 at 8 (with the grouped tail; 41.6 without).  The row groups
+// of skewed matrices keep the compiler's choice (5 blocks): with three matrices
+// in turn 118 us on 4M power-law rows, 123 at 4.
 template <class View> constexpr int spmv_blocks = 5;
 template <> constexpr int spmv_blocks<Hll32SView> = 6;
 template <> constexpr int spmv_blocks<EllView> = 4;
@@ -465,14 +467,13 @@ __device__ __forceinline__ void put_row(int i, double alpha, double a, double be
   y[i] = MODE == 1 ? t : radd(t, rmul(beta, y[i]));
 }
 
-// (4 blocks per SM: 114.1 us on the 4M-row power-law matrix, 115.5 at 5, 118 at
-// 6.)  Rows of the narrow hacks, R per thread, from block `first` on; the rows
+// Rows of the narrow hacks, R per thread, from block `first` on; the rows
 // of wide hacks come from lres (SPLIT 0) or are written by the wide blocks
 // 0 .. first-1 of the same launch (SPLIT 1), which run the split sum and
 // store y themselves: the long rows then overlap the short ones instead of
 // running before them.
 template <int MODE, int SPLIT>
-__global__ void __launch_bounds__(SPMV_T, 4) k_hll_rgroup(Hll32WView A, double alpha, const double *__restrict__ x,
+__global__ void __launch_bounds__(SPMV_T) k_hll_rgroup(Hll32WView A, double alpha, const double *__restrict__ x,
                                                        double beta, double *__restrict__ y) {
   constexpr int R = PSBX_HLL_R;
   const int first = SPLIT ? A.nWChunks : 0;
