@@ -136,6 +136,16 @@ psbx_HllDeviceParams bldHllDeviceParams(unsigned hksize, unsigned rows, unsigned
   return p;
 }
 
+// The kernels that take two adjacent rows in one load (int2, float2, double2)
+// need every hack to start at an even entry.  With the offsets that hack
+// size 32 gives (sums of 32*width from 0) all do; a caller's own arrays may
+// start elsewhere.
+static int even_offsets(const int *hkoffs, size_t n) {
+  for (size_t i = 0; i < n; i++)
+    if (hkoffs[i] & 1) return 0;
+  return 1;
+}
+
 static int hll_copy(void *deviceMat, void *val, int *ja, int *hkoffs, int *irn, int *idiag, bool write, int type) {
   HllDevice *m = (HllDevice *)deviceMat;
   if (!m || m->elemType != type) return SPGPU_UNSUPPORTED;
@@ -152,6 +162,7 @@ static int hll_copy(void *deviceMat, void *val, int *ja, int *hkoffs, int *irn, 
       for (size_t i = 0; i < nr; i++) mx = irn[i] > mx ? irn[i] : mx;
       m->maxRowLen = mx;
     }
+    m->evenOffs = hkoffs ? even_offsets(hkoffs, nh) : 0;
     if (!rc) rc = psbx_hll_index_long(m);
   } else {
     rc = d2h(val, m->cM, as * vsize(type));
@@ -281,6 +292,7 @@ static int coo_to_hll(int nr, int nza, int hacksz, int noffs, int isz, int *irn,
     int mx = 0;
     for (int i = 0; i < nr; i++) mx = irn[i] > mx ? irn[i] : mx;
     m->maxRowLen = mx;
+    m->evenOffs = even_offsets(hoffs, (size_t)noffs + 1);
   }
   if (!rc) rc = sync_stream();
   if (!rc && type == SPGPU_TYPE_DOUBLE) rc = psbx_hll_index_long(m);
@@ -605,6 +617,7 @@ extern "C" int psbx_hll_from_csr_device(void **deviceMat, int rows, int cols, in
   }
   // longest row (the widest hack), for the solver's choice of kernels
   if (!rc && m) m->maxRowLen = (int)res[1];
+  if (!rc && m) m->evenOffs = hksz % 2 == 0;
   if (!rc && m) rc = psbx_hll_index_long(m);
   cudaFree(width);
   cudaFree(irn);

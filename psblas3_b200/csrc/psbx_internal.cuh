@@ -43,6 +43,7 @@ struct HllDevice {
   float *cM32;       // optional FP32 copy of FP64 values (mixed precision)
   int *perm;         // optional storage-row -> matrix-row map (NULL: identity)
   int maxRowLen;     // longest stored row (-1: unknown)
+  int evenOffs;      // every hack starts at an even entry: rows 2k and 2k+1 can be read in pairs
   // hacks wider than longW (hack size 32 only): their row sums are formed
   // before each product (psbx_long_rows32: all products at once into wprod,
   // then a warp per hack adds them in order) and read back from lres by the

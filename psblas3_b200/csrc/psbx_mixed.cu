@@ -452,6 +452,10 @@ extern "C" int psbx_dmixed_cg(void *mat, void *dinv, void *b, void *x, psbx_Solv
       X->elemType != SPGPU_TYPE_DOUBLE || (D && D->elemType != SPGPU_TYPE_DOUBLE))
     return SPGPU_UNSUPPORTED;
   if (opt->istop != 2 || !(delta > 0.0 && delta < 1.0)) return SPGPU_UNSUPPORTED;
+  if (n > 0 && !m->evenOffs) {  // the FP32 product reads rows in pairs
+    psbx_set_error("psbx_dmixed_cg: every hack of the matrix must start at an even entry");
+    return SPGPU_UNSUPPORTED;
+  }
   if (opt->itmax <= 0) {
     opt->iter = 0;
     opt->err = 0.0;

@@ -634,7 +634,7 @@ int psbx_launch_hll_spmv(const HllDevice *m, double alpha, const double *x, doub
     // per thread by default when there are wide hacks (skewed rows)
     const HllView v = hll_view(m);
     if (m->tpr == 2 && m->wideSplit) return launch_tpr2(hll32w_view(v), alpha, x, beta, y, st);
-    if (m->tpr == -2 || m->tpr == 2 || (m->tpr == 0 && v.nLong > 0))
+    if ((m->tpr == -2 || m->tpr == 2 || (m->tpr == 0 && v.nLong > 0)) && m->evenOffs)
       return launch_rgroup(hll32w_view(v), alpha, x, beta, y, st);
     if (v.nLong > 0) return launch_rows(hll32w_view(v), alpha, x, beta, y, st);
     if (hll_short_rows(m)) return launch_rows(hll32s_view(v), alpha, x, beta, y, st);
@@ -871,7 +871,7 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
     PSBX_LAUNCH_CK("k_f32_scale");
     return SPGPU_SUCCESS;
   }
-  if (m->hackSize == 32 && m->maxRowLen >= 0 && m->maxRowLen <= PSBX_SHORT_ROW) {
+  if (m->hackSize == 32 && m->evenOffs && m->maxRowLen >= 0 && m->maxRowLen <= PSBX_SHORT_ROW) {
     const int gp = ((A.rows + 1) / 2 + SPMV_T - 1) / SPMV_T;
     if (beta == 0.0f)
       k_hll_spmv_f32_pairs<1><<<gp, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
