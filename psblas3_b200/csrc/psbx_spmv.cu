@@ -372,35 +372,41 @@ CsrView csr_view(const CsrDevice *m) {
 
 // --------------------------------------------------------------- row kernels
 // MODE 0: y = alpha*acc + beta*y ; MODE 1: beta == 0, y not read.
-// Blocks of SPMV_T per SM that a kernel's registers allow, the fastest of 4, 5,
-// 6 and 8 for each: without a bound the compiler keeps to 32 registers (8
-// blocks) and a group of 8 entries waits in pieces.  27-point HLL 200^3 428 us
-// at 8, 407 at 5 (6.69 TB/s), 410 at 6; 100^3 58 and 51; ELL 101^3 67.6 and
-// 56.2 at 4; 7-point 100^3 HLL 16.4 at 5, 15.3 at 6; ELL 20.5 at 6, 18.5 at 5.
-// The FP32 rows need half the bytes in flight per load: 27-point 100^3 43.1 at
-// 5, 39.3 at 6, 37.0 at 8 (with the grouped tail; 41.6 without).  The row groups
-// of skewed matrices keep the compiler's choice (5 blocks): with three matrices
-// in turn 118 us on 4M power-law rows, 123 at 4.
-template <class View> constexpr int spmv_blocks = 5;
-template <> constexpr int spmv_blocks<Hll32SView> = 6;
-template <> constexpr int spmv_blocks<EllView> = 4;
-template <class View, int MODE>
-__global__ void __launch_bounds__(SPMV_T, spmv_blocks<View>) k_spmv_rows(View A, double alpha, const double *__restrict__ x,
-                                                      double beta, double *__restrict__ y) {
+// BLOCKS: blocks of SPMV_T per SM that the registers allow.  Without a bound
+// the compiler keeps the plain HLL and ELL rows to 32 registers (8 blocks) and
+// a group of 8 entries waits in pieces; the short-row and wide-hack views take
+// 48.  27-point HLL 200^3 428 us at 8, 407 at 5 (6.69 TB/s), 410 at 6; 100^3 58
+// and 51; ELL 101^3 67.6 and 56.2 at 4.  Which instance runs is the launchers'
+// rule (by row length and grid), with the figures there.
+// ONE: a row's last entries one at a time (row_acc), with the compiler's own 32
+// registers (BLOCKS 0: no bound; 1,000,000 rows of 5, hack size 16, 16.4 us, 18.4
+// with the bound of 8).
+template <bool ONE, class View, class T>
+__device__ __forceinline__ double row_sum(const View &A, int s, const T *__restrict__ x) {
+  if constexpr (ONE) return row_dot<true>(A, s, x);
+  else return row_dot(A, s, x);
+}
+template <class View, int MODE, int BLOCKS, bool ONE>
+__global__ void __launch_bounds__(SPMV_T, BLOCKS) k_spmv_rows(View A, double alpha, const double *__restrict__ x,
+                                                              double beta, double *__restrict__ y) {
   const int s = blockIdx.x * SPMV_T + threadIdx.x;
   if (s >= A.rows) return;
-  const double acc = row_dot(A, s, x);
+  const double acc = row_sum<ONE>(A, s, x);
   const int r = out_row(A, s);
   const double t = rmul(alpha, acc);
   y[r] = MODE == 1 ? t : radd(t, rmul(beta, y[r]));
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(SPMV_T, 8) k_hll_spmv_f32(HllViewF A, float alpha, const float *__restrict__ x,
-                                                         float beta, float *__restrict__ y) {
+// (FP32 rows need half the bytes in flight per load: 27-point 100^3 43.1 us at
+// 5 blocks, 39.3 at 6, 37.0 at 8.  One entry at a time the compiler's own 32
+// registers are a better 8 blocks than the bound's: 3,000,000 rows of 16 80.5
+// and 87.0)
+template <int MODE, bool ONE>
+__global__ void __launch_bounds__(SPMV_T, ONE ? 0 : 8) k_hll_spmv_f32(HllViewF A, float alpha, const float *__restrict__ x,
+                                                            float beta, float *__restrict__ y) {
   const int s = blockIdx.x * SPMV_T + threadIdx.x;
   if (s >= A.rows) return;
-  const float acc = (float)row_dot(A, s, x);
+  const float acc = (float)row_sum<ONE>(A, s, x);
   const int r = out_row(A, s);
   const float t = rmulf(alpha, acc);
   y[r] = MODE == 1 ? t : raddf(t, rmulf(beta, y[r]));
@@ -471,7 +477,8 @@ __device__ __forceinline__ void put_row(int i, double alpha, double a, double be
 // of wide hacks come from lres (SPLIT 0) or are written by the wide blocks
 // 0 .. first-1 of the same launch (SPLIT 1), which run the split sum and
 // store y themselves: the long rows then overlap the short ones instead of
-// running before them.
+// running before them.  (Registers as the compiler gives them, 5 blocks per
+// SM: 118 us on 4M power-law rows with three matrices in turn, 123 at 4.)
 template <int MODE, int SPLIT>
 __global__ void __launch_bounds__(SPMV_T) k_hll_rgroup(Hll32WView A, double alpha, const double *__restrict__ x,
                                                        double beta, double *__restrict__ y) {
@@ -610,7 +617,7 @@ static int launch_rgroup(const Hll32WView &A, double alpha, const double *x, dou
   return SPGPU_SUCCESS;
 }
 
-template <class View>
+template <int BLOCKS, bool ONE = false, class View>
 static int launch_rows(const View &A, double alpha, const double *x, double beta, double *y, cudaStream_t st) {
   if (A.rows <= 0) return SPGPU_SUCCESS;
   if (alpha == 0.0) return psbx_launch_scale(A.rows, beta, y, st);
@@ -618,11 +625,48 @@ static int launch_rows(const View &A, double alpha, const double *x, double beta
   if (rc) return rc;
   const int g = (A.rows + SPMV_T - 1) / SPMV_T;
   if (beta == 0.0)
-    k_spmv_rows<View, 1><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    k_spmv_rows<View, 1, BLOCKS, ONE><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
   else
-    k_spmv_rows<View, 0><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    k_spmv_rows<View, 0, BLOCKS, ONE><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
   PSBX_LAUNCH_CK("k_spmv_rows");
   return SPGPU_SUCCESS;
+}
+
+// Grids against the SMs.  (Times below: rows of equal length in bands, queued
+// behind a long kernel, us.)
+static long long rows_blocks(int rows) { return ((long long)rows + SPMV_T - 1) / SPMV_T; }
+static long long rows_waves(long long g, int blocks) {
+  const long long w = (long long)blocks * psbx_ctx().sms;
+  return (g + w - 1) / w;
+}
+// one wave of 4 blocks per SM: latency alone, the loads of a row should be in
+// flight together whatever registers that takes
+static bool small_grid(int rows) { return rows_waves(rows_blocks(rows), 4) <= 1; }
+
+// Hack size 32: 5 blocks per SM (48 registers, 46 for rows beyond
+// PSBX_SHORT_ROW) or 6 (40).  The sixth block is paid for with loads that
+// wait, so it has to save a wave, or the grid has to be so large that the
+// number of rows in flight is what counts:
+//   64,000 rows of 9 entries 5.4 at 5, 6.1 at 6; 110,000 of 16 6.3 and 8.1;
+//   200,000 (782 blocks: 2 waves or 1) of 12 10.2 and 8.2, of 31 18.5 and 16.4;
+//   262,144 (2 waves either way) of 7 7.0 and 6.4, of 12 10.3 and 12.3;
+//   400,000 (3 or 2) of 9 14.3 and 12.3, of 21 22.6 and 20.5;
+//   1,000,000 of 3 14.3 and 12.3, of 12 28.2 and 26.7, of 17 36.2 and 36.9.
+static bool six_blocks(int rows, int longest) {
+  const long long g = rows_blocks(rows), s = psbx_ctx().sms;
+  if (g <= 5 * s) return false;
+  if (longest <= 8) return true;
+  const bool fewer = rows_waves(g, 6) < rows_waves(g, 5);
+  return longest <= PSBX_SHORT_ROW ? fewer || g > 12 * s : fewer && g <= 12 * s;
+}
+static int launch_rows32(const HllDevice *m, const HllView &v, double alpha, const double *x, double beta, double *y,
+                         cudaStream_t st) {
+  if (hll_short_rows(m)) {
+    if (six_blocks(v.rows, m->maxRowLen)) return launch_rows<6>(hll32s_view(v), alpha, x, beta, y, st);
+    return launch_rows<5>(hll32s_view(v), alpha, x, beta, y, st);
+  }
+  if (six_blocks(v.rows, PSBX_SHORT_ROW + 1)) return launch_rows<6>(hll32_view(v), alpha, x, beta, y, st);
+  return launch_rows<5>(hll32_view(v), alpha, x, beta, y, st);
 }
 
 int psbx_launch_hll_spmv(const HllDevice *m, double alpha, const double *x, double beta, double *y,
@@ -636,11 +680,18 @@ int psbx_launch_hll_spmv(const HllDevice *m, double alpha, const double *x, doub
     if (m->tpr == 2 && m->wideSplit) return launch_tpr2(hll32w_view(v), alpha, x, beta, y, st);
     if ((m->tpr == -2 || m->tpr == 2 || (m->tpr == 0 && v.nLong > 0)) && m->evenOffs)
       return launch_rgroup(hll32w_view(v), alpha, x, beta, y, st);
-    if (v.nLong > 0) return launch_rows(hll32w_view(v), alpha, x, beta, y, st);
-    if (hll_short_rows(m)) return launch_rows(hll32s_view(v), alpha, x, beta, y, st);
-    return launch_rows(hll32_view(v), alpha, x, beta, y, st);
+    if (v.nLong > 0) return launch_rows<5>(hll32w_view(v), alpha, x, beta, y, st);
+    return launch_rows32(m, v, alpha, x, beta, y, st);
   }
-  return launch_rows(hll_view(m), alpha, x, beta, y, st);
+  // other hack sizes: a column's stride is not a constant, and the predicated
+  // tails cost short rows of large grids more instructions than they save
+  // waiting: 1,000,000 rows of 1 entry 8.2 against 11.8, of 5 16.3 and 20.6, of
+  // 13 32.8 and 34.8; 64,000 rows of 13 9.1 and 6.4,
+  // 150,000 of 9 8.7 and 7.2; 1,000,000 of 27 64.7 and
+  // 58.7 (61.1 at 5 blocks).
+  if (m->maxRowLen >= 0 && m->maxRowLen <= PSBX_SHORT_ROW && !small_grid(m->rows))
+    return launch_rows<0, true>(hll_view(m), alpha, x, beta, y, st);
+  return launch_rows<4>(hll_view(m), alpha, x, beta, y, st);
 }
 
 // ------------------------------------------------- host-buffer SpMV
@@ -707,8 +758,7 @@ static int launch_hll_rows_range(const HllDevice *m, int r0, int nr, double alph
   v.irn += r0;
   v.hkoffs += r0 / 32;
   v.rows = nr;
-  if (hll_short_rows(m)) return launch_rows(hll32s_view(v), alpha, x, beta, y + r0, st);
-  return launch_rows(hll32_view(v), alpha, x, beta, y + r0, st);
+  return launch_rows32(m, v, alpha, x, beta, y + r0, st);
 }
 
 extern "C" int psbx_hll_spmv_host(void *deviceMat, double alpha, const double *x, double beta, double *y,
@@ -817,11 +867,14 @@ extern "C" int psbx_hll_spmv_host(void *deviceMat, double alpha, const double *x
   return SPGPU_SUCCESS;
 }
 
-// FP32, hack size 32, short rows: two adjacent rows per thread (entry j of both
-// is one float2 and one int2, 256 bytes per warp load where one row moves
-// 128), the sums of k_hll_spmv_f32 bit for bit.  7-point 100^3: 16.4 us, one
-// row per thread 20.5; the 27-point rows are the other way round (64 us
-// against 39): a pair holds more loads in flight than the registers take.
+// FP32, hack size 32, rows of 6 or 7 entries: two adjacent rows per thread
+// (entry j of both is one float2 and one int2, 256 bytes per warp load where
+// one row moves 128), the sums of k_hll_spmv_f32 bit for bit.  Against one row
+// per thread, rows of 7: 16.5 and 18.4 us on 1,000,000, 7.1 and 7.9 on 200,000,
+// the same on 64,000.  Such a row is just under a group of 8; a full group or
+// a few entries are the other way round (of 8 45.1 and 34.8 on 3,000,000, of 9
+// 67.5 and 39.7, of 4 36.7 and 28.7, of 1 31.9 and 18.5): the pair's second
+// row and its empty slots are issued all the same.
 template <int MODE>
 __global__ void __launch_bounds__(SPMV_T, 5) k_hll_spmv_f32_pairs(HllViewF A, float alpha, const float *__restrict__ x,
                                                                float beta, float *__restrict__ y) {
@@ -844,8 +897,18 @@ __global__ void __launch_bounds__(SPMV_T, 5) k_hll_spmv_f32_pairs(HllViewF A, fl
 int psbx_launch_ell_spmv(const EllDevice *m, double alpha, const double *x, double beta, double *y,
                          cudaStream_t st) {
   if (m->dataType != SPGPU_TYPE_DOUBLE) return SPGPU_UNSUPPORTED;
-  if (m->maxRowSize <= PSBX_SHORT_ROW) return launch_rows(ells_view(ell_view(m)), alpha, x, beta, y, st);
-  return launch_rows(ell_view(m), alpha, x, beta, y, st);
+  const EllView v = ell_view(m);
+  const int longest = m->maxRowSize;
+  if (longest > PSBX_SHORT_ROW) return launch_rows<4>(v, alpha, x, beta, y, st);
+  // short rows as predicated groups of 8 where the last group is nearly full,
+  // or the grid small: 1,000,000 rows of 7 18.4 us, one entry at a time 20.5; of
+  // 13 30.8 and 32.7; of 9 26.6 and 24.6; of 5 16.4 and 16.3 (262,144: 7.2 and
+  // 6.1); of 1 14.4 and 8.1; 64,000 rows of 9 6.1 and 6.1, of 13 6.2 and 8.2, of 4
+  // 4.1 and 5.1, of 2 5.2 and 4.1
+  const int unused = (longest + 7) / 8 * 8 - longest;
+  if (4 * unused <= longest || (longest >= 4 && small_grid(v.rows)))
+    return launch_rows<5>(ells_view(v), alpha, x, beta, y, st);
+  return launch_rows<0, true>(v, alpha, x, beta, y, st);
 }
 
 __global__ void k_f32_scale(int n, float beta, float *__restrict__ y) {
@@ -871,7 +934,7 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
     PSBX_LAUNCH_CK("k_f32_scale");
     return SPGPU_SUCCESS;
   }
-  if (m->hackSize == 32 && m->evenOffs && m->maxRowLen >= 0 && m->maxRowLen <= PSBX_SHORT_ROW) {
+  if (m->hackSize == 32 && m->evenOffs && (m->maxRowLen == 6 || m->maxRowLen == 7)) {
     const int gp = ((A.rows + 1) / 2 + SPMV_T - 1) / SPMV_T;
     if (beta == 0.0f)
       k_hll_spmv_f32_pairs<1><<<gp, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
@@ -881,10 +944,21 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
     return SPGPU_SUCCESS;
   }
   const int g = (A.rows + SPMV_T - 1) / SPMV_T;
-  if (beta == 0.0f)
-    k_hll_spmv_f32<1><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
-  else
-    k_hll_spmv_f32<0><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  // short rows of other hack sizes one entry at a time at the end, as in FP64:
+  // 1,000,000 rows of 2 10.1 us against 12.3, of 13 29.5 and 30.7; of 27 59.5 and
+  // 54.9; not rows of 3 (13.3 and 12.2), nor of 4 on a small grid (64,000 5.1 and 4.2)
+  const int longest = m->maxRowLen;
+  if (m->hackSize != 32 && longest >= 0 && longest <= PSBX_SHORT_ROW && longest != 3 &&
+      !(longest == 4 && small_grid(A.rows))) {
+    if (beta == 0.0f)
+      k_hll_spmv_f32<1, true><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    else
+      k_hll_spmv_f32<0, true><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  } else if (beta == 0.0f) {
+    k_hll_spmv_f32<1, false><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  } else {
+    k_hll_spmv_f32<0, false><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  }
   PSBX_LAUNCH_CK("k_hll_spmv_f32");
   return SPGPU_SUCCESS;
 }
@@ -893,12 +967,12 @@ int psbx_launch_hll_spmv_f32(const HllDevice *m, float alpha, const float *x, fl
 // the row sum is formed like the FP32 HLL one -- every product of two floats
 // is exact in FP64, the products are added in FP64 in stored order and the
 // sum is rounded to FP32 once -- then y = alpha*sum + beta*y in FP32.
-template <int MODE>
-__global__ void __launch_bounds__(SPMV_T, 8) k_ell_spmv_f32(EllViewF A, float alpha, const float *__restrict__ x,
-                                                         float beta, float *__restrict__ y) {
+template <int MODE, bool ONE>
+__global__ void __launch_bounds__(SPMV_T, ONE ? 0 : 8) k_ell_spmv_f32(EllViewF A, float alpha, const float *__restrict__ x,
+                                                            float beta, float *__restrict__ y) {
   const int r = blockIdx.x * SPMV_T + threadIdx.x;
   if (r >= A.rows) return;
-  const float acc = (float)row_dot(A, r, x);
+  const float acc = (float)row_sum<ONE>(A, r, x);
   const float t = rmulf(alpha, acc);
   y[r] = MODE == 1 ? t : raddf(t, rmulf(beta, y[r]));
 }
@@ -920,10 +994,16 @@ int psbx_launch_ell_spmv_f32(const EllDevice *m, float alpha, const float *x, fl
     return SPGPU_SUCCESS;
   }
   const int g = (A.rows + SPMV_T - 1) / SPMV_T;
-  if (beta == 0.0f)
-    k_ell_spmv_f32<1><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
-  else
-    k_ell_spmv_f32<0><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  if (m->maxRowSize <= PSBX_SHORT_ROW) {  // as the FP32 HLL rows of a hack size other than 32
+    if (beta == 0.0f)
+      k_ell_spmv_f32<1, true><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+    else
+      k_ell_spmv_f32<0, true><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  } else if (beta == 0.0f) {
+    k_ell_spmv_f32<1, false><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  } else {
+    k_ell_spmv_f32<0, false><<<g, SPMV_T, 0, st>>>(A, alpha, x, beta, y);
+  }
   PSBX_LAUNCH_CK("k_ell_spmv_f32");
   return SPGPU_SUCCESS;
 }

@@ -56,3 +56,46 @@ def test_row_forms(psb, n, longest, alpha, beta):
         X, Y = psb.DVect.bld(x32), psb.DVect.bld(y32)
         A.spmv(alpha, X, beta, Y)
         assert np.array_equal(Y.get_vect(), ref32)
+
+
+def _bands(n, longest, seed):
+    """Rows of 0 .. longest neighbouring columns, the longest row among them."""
+    rng = np.random.default_rng(seed)
+    k = rng.integers(0, longest + 1, n)
+    k[n // 2] = longest
+    irp = np.concatenate([[1], 1 + np.cumsum(k)]).astype(np.int32)
+    first = rng.integers(1, n - longest + 2, n)
+    ja = (np.repeat(first, k) + np.arange(irp[-1] - 1) - np.repeat(irp[:-1] - 1, k)).astype(np.int32)
+    return irp, ja, rng.standard_normal(len(ja))
+
+
+@pytest.mark.parametrize("longest", [1, 3, 4, 6, 7, 8, 9, 13, 16, 21])
+@pytest.mark.parametrize("blocks", [4, 5, 6, 10, 12])
+def test_forms_at_grid_lines(psb, blocks, longest):
+    """The forms of the row products change with the row length and the grid
+    (4, 5, 6, 10 and 12 blocks of 256 rows per SM): one row past each line,
+    hack sizes 32 and 16, ELL, FP64 and FP32."""
+    from psblas3_b200._lib import lib
+    n = 256 * blocks * lib.getGPUMultiProcessors() + 1
+    irp, ja, va = _bands(n, longest, 7)
+    rng = np.random.default_rng(5)
+    x, y0 = rng.uniform(-1, 1, (2, n))
+    ref = O.csr_csmv(irp, ja, va, -0.5, x, 2.0, y0.copy())
+    v32, x32, y32 = va.astype(np.float32), x.astype(np.float32), y0.astype(np.float32)
+    s = O.csr_csmv(irp, ja, v32.astype(np.float64), 1.0, x32.astype(np.float64), 0.0, np.zeros(n)).astype(np.float32)
+    ref32 = np.float32(-0.5) * s + np.float32(2.0) * y32
+    ia, _, _ = gen.csr_to_coo(irp, ja, va)
+    import torch
+    d = [torch.from_numpy(a).cuda() for a in (irp, ja, va)]
+    torch.cuda.synchronize()
+    mats = [psb.HllMat.from_csr_device(n, n, len(ja), *(t.data_ptr() for t in d), hk) for hk in (32, 16)]
+    mats.append(psb.EllMat.from_coo_gpu(n, ia, ja, va))
+    for A in mats:
+        X, Y = psb.DVect.bld(x), psb.DVect.bld(y0)
+        psb.psb_spmm(-0.5, A, X, 2.0, Y)
+        assert np.array_equal(Y.get_vect(), ref)
+    for A in mats[:2]:
+        A.make_single()
+        X, Y = psb.DVect.bld(x32), psb.DVect.bld(y32)
+        A.spmv(-0.5, X, 2.0, Y)
+        assert np.array_equal(Y.get_vect(), ref32)
