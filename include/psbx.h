@@ -444,7 +444,8 @@ int psbx_DefaultSolverOptions(psbx_SolverOptions *opt);
  * device; the host reads a status word once per captured batch of
  * iterations -- or once per solve: CG and BiCGSTAB of systems whose vectors
  * fit the SMs' shared memory (about 700,000 / 510,000 rows, no wide hacks,
- * itmax <= 100000) run as one cooperative kernel.  Returns 0 (converged or
+ * itmax <= 100000, and no run of rows so long that one SM would hold the others
+ * up) run as one cooperative kernel.  Returns 0 (converged or
  * itmax reached, as the reference), or an error code (PSBX_TIMEOUT: a wait
  * between that kernel's blocks ran past its bound); opt->iter and opt->err
  * are filled like psb_krylov's iter and err. */

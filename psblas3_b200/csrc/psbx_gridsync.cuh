@@ -24,8 +24,8 @@
 
 #include "psbx_internal.cuh"
 
-#define GS_MAXV 6                        // 8-byte values a reduction carries: 2 per sum, 1 per max
-#define GS_MAXWARPS 32
+#define GS_MAXV 8                        // 8-byte values a reduction carries: 2 per sum, 1 per max
+#define GS_MAXWARPS 16                   // warps of a block
 #define GS_WAIT_NS 10000000000ull        // 10 s: far beyond any phase, and finite
 
 // Shared memory of the reductions of one block.
@@ -105,7 +105,7 @@ __device__ __forceinline__ void grid_reduce(GridSync &g, dd_t (&s)[S > 0 ? S : 1
   static_assert(NV <= GS_MAXV && GS_MAXV <= GS_SLOT, "values per reduction");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int par = (int)(g.seq & 1);
-  GsShared &sh = *g.sh;
+  GsShared &sh = *g.sh;  // (its arrays hold GS_MAXWARPS warps: the launch bound of the kernels that use it)
   auto from_warps = [&]() {
 #pragma unroll
     for (int k = 0; k < S; k++)

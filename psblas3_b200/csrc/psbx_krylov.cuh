@@ -24,8 +24,9 @@ struct KState {
 
 // One-kernel CG / BiCGSTAB (psbx_persist.cu).  persist_fits: whether the
 // system is in its range; persist_solve: runs the solve and fills opt like
-// the drivers, or leaves *ran 0 with nothing done (itmax beyond its range, or
-// a device that cannot hold the kernel's blocks at once).
+// the drivers, or leaves *ran 0 with nothing done (itmax beyond its range, rows
+// that would keep one block busy while the others wait, or a device that cannot
+// hold the kernel's blocks at once).
 bool persist_fits(const HllView &A, bool bicg);
 bool persist_fits(const EllView &A, bool bicg);
 bool persist_fits(const CsrView &A, bool bicg);

@@ -29,14 +29,18 @@
 #include <string.h>
 
 #define PS_MAXT 512   // (1024 threads at 64 registers: 3 to 15 % slower)
+static_assert(PS_MAXT / 32 <= GS_MAXWARPS, "warps of a block");
 #define PS_SMEM (212 * 1024)  // dynamic shared memory of a block at most
-// Largest itmax taken here: a solve that never converges then ends within
-// about a second (the kernel-per-step drivers take the rest).
+// Largest itmax taken here (the kernel-per-step drivers take the rest): the
+// host waits for the one kernel, so a solve that never converges should end
+// in seconds.  100,000 iterations are 1.8 s (CG) and 3.4 s (BiCGSTAB) on 512,000
+// rows of the 7-point operators, more by the unstaged entries that ps_limit lets
+// through.
 #define PS_MAXIT 100000
 
 struct PsOut {         // the solve's result, in page-locked host memory
   double errnum, errden;
-  int itx, timeout;
+  int itx, timeout, declined;
 };
 
 // Entries of storage row s: the j-th at v[j*st], column p[j*st].
@@ -68,7 +72,42 @@ struct PsArgs {
   int mat_entries;     // matrix entries a block's shared memory holds
   int itmax, istop;
   double eps;
+  double most, per_mean, per_longest;  // what a block may read through L2 (PsLoad)
 };
+
+// What a block's products read through L2, in quarters of an entry: the
+// entries of its slices that are not staged, weighted.  A block's SM reads
+// them alone in every iteration, so the solve is as slow as the fullest block
+// -- long rows side by side, or rows too many for the staging area -- while
+// the kernel-per-step drivers spread the same rows over all SMs.
+//   1.5 for rows of more than 8 entries (a slice's average) that are held one
+//     after the other (CSR): a warp's loads touch a line per lane, more than the
+//     L1 that the staging area leaves can hold;
+//   else 0.25 + 0.75 * lines / lanes, for the lines of x that a gather touches
+//     (seen at the middle entry of each row): 0.3 for a stencil, 1 at random.
+struct PsLoad {
+  unsigned long long cost, entries;  // weighted and unstaged; all
+  int longest;
+};
+
+// Most a block may carry for the kernel to go on: a + m * (entries of an
+// average block) + r * (longest row); the drivers' own time grows with
+// both.  Fitted to 593 solves (length-sorted power-law rows up to 128 entries,
+// rows that are long in one part of a banded matrix, random rows, 7- and
+// 27-point grids; 60,000 to 690,000 rows; CSR, ELL, HLL), each timed both ways.  us an
+// iteration here and with a kernel per step: CG, CSR, length-sorted rows up to 69
+// entries on 480,000 rows (144,000 entries unstaged) 402 and 70; BiCGSTAB 801 and
+// 115; CG, HLL, 27-point 84^3 72 and 56, 67^3 30 and 41; CG, 7-point 88^3 (31,000 unstaged)
+// 22 and 34.  With the staging area beyond PS_SMEM_L1 the SM's L1 has only
+// 28 KB left for the gathers and their cost doubles (200,000 rows, BiCGSTAB: 50 us
+// at 184 KB, 98 at 190).
+#define PS_SMEM_L1 (188 * 1024)
+static void ps_limit(PsArgs &P, size_t smem) {
+  const bool l1 = smem <= PS_SMEM_L1;
+  P.most = l1 ? 20480.0 : 18432.0;
+  P.per_mean = l1 ? 0.75 : 0.125;
+  P.per_longest = l1 ? 320.0 : 128.0;
+}
 
 // A block's rows and their data in shared memory.
 struct Blk {
@@ -132,6 +171,36 @@ __device__ __forceinline__ void each_row(const Blk &B, const View &A, F &&f) {
   for (int k = threadIdx.x >> 5; k < B.ns; k += nw) {
     const int l = k * 32 + lane, s = B.s0 + l;
     if (s < A.rows) f(l, out_row(A, s));
+  }
+}
+
+// The load of a block whose rows are staged.  (A loop of its own, not
+// unrolled: inside the staging loop it cost HLL's CG 2 to 20 % an iteration
+// through the register allocation of the products.)
+template <class View>
+__device__ __forceinline__ void slice_loads(const Blk &B, const View &A, PsLoad &load) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll 1
+  for (int k = warp; k < B.ns; k += nw) {
+    const int l = k * 32 + lane, s = B.s0 + l, o = B.off[k], n = B.len[l];
+    const unsigned e = __reduce_add_sync(0xffffffffu, (unsigned)n);
+    const int w = __reduce_max_sync(0xffffffffu, n);
+    unsigned long long cost = 0;
+    if (o < 0) {
+      RowPtr r = {nullptr, nullptr, 0, 0};
+      if (n > 0) r = row_ptr(A, s);
+      const int line = n > 0 ? ld_ro(r.p + (size_t)(n / 2) * r.st) >> 4 : -1;
+      const unsigned lanes = __popc(__ballot_sync(0xffffffffu, n > 0));
+      const unsigned first = __ffs(__match_any_sync(0xffffffffu, line)) - 1;
+      const unsigned lines = __popc(__ballot_sync(0xffffffffu, n > 0 && (int)first == lane));
+      const bool by_row = __any_sync(0xffffffffu, r.st == 1);
+      cost = by_row && e > 8 * lanes ? 6ull * e : e + 3ull * e * lines / lanes;
+    }
+    if (lane == 0) {
+      atomicAdd(&load.entries, (unsigned long long)e);
+      atomicAdd(&load.cost, cost);
+      atomicMax(&load.longest, w);
+    }
   }
 }
 
@@ -207,15 +276,27 @@ __global__ void __launch_bounds__(PS_MAXT, 1) k_persist(View A, PsArgs P) {
   B.sj = (int *)(B.sv + P.mat_entries);
   B.len = B.sj + P.mat_entries;
   B.off = B.len + nloc;
-  if (threadIdx.x == 0) gsh.bad = 0;
+  __shared__ PsLoad load;
+  if (threadIdx.x == 0) {
+    gsh.bad = 0;
+    load.cost = load.entries = 0;
+    load.longest = 0;
+  }
   stage(B, A, P.mat_entries);
+  slice_loads(B, A, load);
+  __syncthreads();
   GridSync G = {P.slots, &gsh, 0, (int)gridDim.x};
   const bool norms = P.istop == 1;  // the stop test needs max|r| and max|x|
 
   Conv c = {0, 0, 0, 0, 0, 0, 0};
   {
-    dd_t s[1] = {{0.0, 0.0}};
-    double m[2] = {0.0, 0.0};
+    dd_t s[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    double m[4] = {0.0, 0.0, 0.0, 0.0};
+    if (threadIdx.x == 0) {
+      s[1].s = (double)load.entries;
+      m[2] = (double)load.cost;
+      m[3] = (double)load.longest;
+    }
     each_row(B, A, [&](int l, int i) {
       const double bi = P.b[i];
       lx[l] = P.x[i];
@@ -229,10 +310,14 @@ __global__ void __launch_bounds__(PS_MAXT, 1) k_persist(View A, PsArgs P) {
         m[1] = fmax(m[1], t);
       }
     });
-    grid_reduce<1, 2, false>(G, s, m);
+    grid_reduce<2, 4, false>(G, s, m);
     c.bn2 = sqrt(dd_value(s[0]));
     c.bni = m[0];
     c.ani = m[1];
+    if (!gsh.bad && 0.25 * m[2] > P.most + P.per_mean * dd_value(s[1]) / gridDim.x + P.per_longest * m[3]) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) P.out->declined = 1;
+      return;  // nothing written: the drivers take the solve
+    }
   }
   bool restarted = false;
   int r0set = 0;
@@ -460,6 +545,7 @@ static int run(const View &A, const double *dinv, const double *b, double *x, ps
   P.itmax = opt->itmax;
   P.istop = opt->istop;
   P.eps = opt->eps;
+  ps_limit(P, smem);
   memset(P.out, 0, sizeof(PsOut));
   e = cudaMemsetAsync(ws, 0, GS_BYTES(g), st);
   View Av = A;
@@ -475,6 +561,7 @@ static int run(const View &A, const double *dinv, const double *b, double *x, ps
   cudaFreeAsync(ws, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return psbx_cuda_status(e, "k_persist");
+  if (P.out->declined && !P.out->timeout) return SPGPU_SUCCESS;
   *ran = 1;
   if (P.out->timeout) {
     psbx_set_error("psbx_dkrylov: a wait between the blocks of the solve ran past its bound");

@@ -117,6 +117,26 @@ def test_upper_end(psb):
         assert np.linalg.norm(r) <= 2e-8 * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("fmt", ["CSR", "HLL16", "ELL"])
+def test_uneven_rows_go_to_the_drivers(psb, fmt):
+    """Rows in order of length: the first blocks would hold most of the entries
+    and read them alone, so the kernel declines and x is the drivers'; the same
+    rows shuffled, and a grid with as many unstaged entries, stay in it."""
+    n = 300_000
+    irp, ja, va = gen.powerlaw_spd(n, kmax=40, seed=4)
+    b = np.random.default_rng(8).uniform(-1, 1, n)
+    sirp, sja, sva = gen.sort_rows_by_length(irp, ja, va)[:3]
+    A = _matrix(psb, fmt, sirp, sja, sva)
+    it1, err1, x1, l1 = _solve(psb, A, "CG", b, 5000)
+    it2, err2, x2, l2 = _solve(psb, A, "CG", b, GENERAL)
+    assert l1 == l2 + 1  # the kernel that declined, then the same launches
+    assert (it1, err1) == (it2, err2) and np.array_equal(x1, x2)
+    if fmt != "ELL":  # (padded to the longest row everywhere)
+        assert _solve(psb, _matrix(psb, fmt, irp, ja, va), "CG", b, 5000)[3] == 1
+    irp, ja, va = gen.poisson7(66)
+    assert _solve(psb, _matrix(psb, fmt, irp, ja, va), "CG", b[:66 ** 3], 5000)[3] == 1
+
+
 @pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
 def test_breakdown_and_itmax(psb, method):
     """A breakdown at every restart ends at itmax, as in the general path; so
