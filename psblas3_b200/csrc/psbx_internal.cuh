@@ -499,8 +499,12 @@ struct EllSView : EllView {};  // the same for ELL
 // allocation below 2^31 entries, as psb_ipk_ does).  The U index and value
 // loads of a group are issued before its U gathers, the gathers before the
 // adds, so each thread keeps 2U streaming loads in flight.
-// ONE: the entries left over one at a time instead of in groups of four.
-template <class VT, class XT, int U, int STRIDE, bool ONE = false>
+// TAIL: the entries left over in groups of four (the solvers' kernels); in
+// groups of four but a last entry alone (the products: a whole group for it cost
+// them 3 to 10 % on rows of 21, 25 and 29 entries, while the solvers' short rows
+// lost 4 % by it); or one at a time.
+enum { TAIL_GROUPS, TAIL_LAST, TAIL_ONE };
+template <class VT, class XT, int U, int STRIDE, int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_acc(const VT *__restrict__ vp, const int *__restrict__ jp, int stride, int n,
                                           const XT *__restrict__ xb) {
   const int st = STRIDE > 0 ? STRIDE : stride;
@@ -523,7 +527,7 @@ __device__ __forceinline__ double row_acc(const VT *__restrict__ vp, const int *
 #pragma unroll
     for (int u = 0; u < U; u++) acc = radd(acc, rmul((double)v[u], (double)xv[u]));
   }
-  if (ONE) {
+  if (TAIL == TAIL_ONE) {
     for (; j < n; j++) {
       const int c = ld_stream(jp + j * st);
       const VT v = ld_stream(vp + j * st);
@@ -531,13 +535,11 @@ __device__ __forceinline__ double row_acc(const VT *__restrict__ vp, const int *
     }
     return acc;
   }
-  // the tail in predicated groups of TU (one entry at a time it was a chain of
-  // up to U - 1 more pairs of round trips, as long again as a 27-entry row),
-  // but a last entry alone: a whole group for it cost 3 to 10 % on rows of 21,
-  // 25 and 29 entries
+  // the tail in predicated groups of TU: one entry at a time it was a chain of
+  // up to U - 1 more pairs of round trips, as long again as a 27-entry row
   constexpr int TU = U < 4 ? U : 4;
   for (; j < n; j += TU) {
-    if (j + 1 == n) {
+    if (TAIL == TAIL_LAST && j + 1 == n) {
       const int c = ld_stream(jp + j * st);
       const VT v = ld_stream(vp + j * st);
       return radd(acc, rmul((double)v, (double)ld_ro(xb + c)));
@@ -650,9 +652,10 @@ __device__ __forceinline__ double row_dot(const Hll32SView &A, int s, const doub
   return row_acc_p<double, double, 8, 32>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base, A.base);
 }
 
+template <int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_dot(const Hll32View &A, int s, const double *__restrict__ x) {
   const int off = ld_ro(A.hkoffs + (s >> 5)) + (s & 31);
-  return row_acc<double, double, 8, 32>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base);
+  return row_acc<double, double, 8, 32, TAIL>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base);
 }
 
 __device__ __forceinline__ double row_dot(const Hll32WView &A, int s, const double *__restrict__ x) {
@@ -666,34 +669,34 @@ __device__ __forceinline__ double row_dot(const Hll32WView &A, int s, const doub
   return row_acc_p<double, double, 8, 32>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base, A.base);
 }
 
-template <bool ONE = false>
+template <int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_dot(const HllView &A, int s, const double *__restrict__ x) {
   const int h = s / A.hksz;
   const int off = ld_ro(A.hkoffs + h) + (s - h * A.hksz);
-  return row_acc<double, double, 8, 0, ONE>(A.val + off, A.ja + off, A.hksz, ld_ro(A.irn + s), x - A.base);
+  return row_acc<double, double, 8, 0, TAIL>(A.val + off, A.ja + off, A.hksz, ld_ro(A.irn + s), x - A.base);
 }
 
-template <bool ONE = false>
+template <int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_dot(const HllViewF &A, int s, const float *__restrict__ x) {
   const int h = s / A.hksz;
   const int off = ld_ro(A.hkoffs + h) + (s - h * A.hksz);
   if (A.hksz == 32)
-    return row_acc<float, float, 8, 32, ONE>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base);
-  return row_acc<float, float, 8, 0, ONE>(A.val + off, A.ja + off, A.hksz, ld_ro(A.irn + s), x - A.base);
+    return row_acc<float, float, 8, 32, TAIL>(A.val + off, A.ja + off, 32, ld_ro(A.irn + s), x - A.base);
+  return row_acc<float, float, 8, 0, TAIL>(A.val + off, A.ja + off, A.hksz, ld_ro(A.irn + s), x - A.base);
 }
 
-template <bool ONE = false>
+template <int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_dot(const EllView &A, int r, const double *__restrict__ x) {
-  return row_acc<double, double, 8, 0, ONE>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base);
+  return row_acc<double, double, 8, 0, TAIL>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base);
 }
 
 __device__ __forceinline__ double row_dot(const EllSView &A, int r, const double *__restrict__ x) {
   return row_acc_p<double, double, 8, 0>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base, A.base);
 }
 
-template <bool ONE = false>
+template <int TAIL = TAIL_GROUPS>
 __device__ __forceinline__ double row_dot(const EllViewF &A, int r, const float *__restrict__ x) {
-  return row_acc<float, float, 8, 0, ONE>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base);
+  return row_acc<float, float, 8, 0, TAIL>(A.val + r, A.ja + r, A.pitch, ld_ro(A.irn + r), x - A.base);
 }
 
 __device__ __forceinline__ double row_dot(const CsrView &A, int r, const double *__restrict__ x) {

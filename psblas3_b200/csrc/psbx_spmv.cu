@@ -383,8 +383,17 @@ CsrView csr_view(const CsrDevice *m) {
 // with the bound of 8).
 template <bool ONE, class View, class T>
 __device__ __forceinline__ double row_sum(const View &A, int s, const T *__restrict__ x) {
-  if constexpr (ONE) return row_dot<true>(A, s, x);
-  else return row_dot(A, s, x);
+  return row_dot<ONE ? TAIL_ONE : TAIL_LAST>(A, s, x);
+}
+// (these read a row's last entries as one predicated group)
+template <bool ONE> __device__ __forceinline__ double row_sum(const Hll32SView &A, int s, const double *__restrict__ x) {
+  return row_dot(A, s, x);
+}
+template <bool ONE> __device__ __forceinline__ double row_sum(const Hll32WView &A, int s, const double *__restrict__ x) {
+  return row_dot(A, s, x);
+}
+template <bool ONE> __device__ __forceinline__ double row_sum(const EllSView &A, int s, const double *__restrict__ x) {
+  return row_dot(A, s, x);
 }
 template <class View, int MODE, int BLOCKS, bool ONE>
 __global__ void __launch_bounds__(SPMV_T, BLOCKS) k_spmv_rows(View A, double alpha, const double *__restrict__ x,
