@@ -1738,11 +1738,6 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
     psbx_count_launch();
   }
 
-  const int gp = bicg ? resident_grid(k_bcg_p, grid) : resident_grid(k_cg_p, grid);
-  const int gs = resident_grid(k_bcg_s, grid);
-  const int g1 = bicg ? resident_grid(k_bcg_spmv1<View>, grid) : resident_grid(k_cg_spmv<View>, grid);
-  const int g2 = resident_grid(k_bcg_spmv2<View>, grid);
-  const int gu = bicg ? resident_grid(k_bcg_update, grid) : resident_grid(k_cg_update, grid);
   // one captured batch of KGRAPH_ITERS iterations (kept from an earlier call
   // with the same arguments, or captured now)
   cudaGraph_t graph = nullptr;
@@ -1752,6 +1747,11 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "BeginCapture");
   }
   if (!rc && !gexec) {
+    const int gp = bicg ? resident_grid(k_bcg_p, grid) : resident_grid(k_cg_p, grid);
+    const int gs = bicg ? resident_grid(k_bcg_s, grid) : 0;
+    const int g1 = bicg ? resident_grid(k_bcg_spmv1<View>, grid) : resident_grid(k_cg_spmv<View>, grid);
+    const int g2 = bicg ? resident_grid(k_bcg_spmv2<View>, grid) : 0;
+    const int gu = bicg ? resident_grid(k_bcg_update, grid) : resident_grid(k_cg_update, grid);
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       if (!bicg) {
         k_cg_p<<<gp, KT, 0, st>>>(S, n, v3, v0);
@@ -1794,14 +1794,15 @@ static int solve(const View &A, bool bicg, const double *dinv, const double *b, 
   };
 
   if (!rc) rc = fetch();
+  const int gi = bicg ? resident_grid(k_bcg_init<View>, grid) : resident_grid(k_cg_init<View>, grid);
   // restart loop (psb_dcg.F90:218-225 / psb_dcgstab.f90:226-237)
   while (!rc) {
     if (hS->itx >= opt->itmax) break;
     if ((rc = psbx_long_rows(A, x, nullptr, st))) break;
     if (!bicg)
-      k_cg_init<View><<<resident_grid(k_cg_init<View>, grid), KT, 0, st>>>(A, S, b, x, dinv, v2, v3, part, ticket, grid);
+      k_cg_init<View><<<gi, KT, 0, st>>>(A, S, b, x, dinv, v2, v3, part, ticket, grid);
     else
-      k_bcg_init<View><<<resident_grid(k_bcg_init<View>, grid), KT, 0, st>>>(A, S, b, x, v1, v0, part, ticket, grid);
+      k_bcg_init<View><<<gi, KT, 0, st>>>(A, S, b, x, v1, v0, part, ticket, grid);
     psbx_count_launch(1 + long_launch(A));
     if ((rc = fetch())) break;
     if (hS->status == ST_DONE) break;
@@ -1869,10 +1870,11 @@ static int solve_fcg(const View &A, const double *dinv, const double *b, double 
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) rc = psbx_cuda_status(e, "BeginCapture");
   if (!rc) {
+    const int g1 = resident_grid(k_fcg_spmv<View>, grid), gu = resident_grid(k_fcg_update, grid);
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       psbx_long_rows(A, v, &S->status, st);
-      k_fcg_spmv<View><<<resident_grid(k_fcg_spmv<View>, grid), KT, 0, st>>>(A, S, v, r, q, w, part, ticket, grid);
-      k_fcg_update<<<resident_grid(k_fcg_update, grid), KT, 0, st>>>(S, n, w, dinv, v, d, q, x, r, part, ticket, grid);
+      k_fcg_spmv<View><<<g1, KT, 0, st>>>(A, S, v, r, q, w, part, ticket, grid);
+      k_fcg_update<<<gu, KT, 0, st>>>(S, n, w, dinv, v, d, q, x, r, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");
@@ -1965,13 +1967,16 @@ static int solve_gmres(const View &A, const double *dinv, const double *b, doubl
     psbx_long_rows(A, x, &S->status, st);
     k_gm_resid<View><<<grid, KT, 0, st>>>(A, S, G, b, x, Vk(0), part, ticket, grid);
     per_graph += 1 + long_launch(A);
+    // (asked once: nl*nl/2 queries during the capture were 3 % of a small solve)
+    const int g1 = resident_grid(k_gm_spmv<View>, grid), gm = resident_grid(k_gm_mgs, grid),
+              gn = resident_grid(k_gm_norm, grid);
     for (int i = 1; i <= nl; i++) {
       k_gm_next<<<grid, KT, 0, st>>>(S, n, i == 1 ? Vk(0) : w, Vk(i - 1), dinv, w1);
       psbx_long_rows(A, w1, &S->status, st);
-      k_gm_spmv<View><<<resident_grid(k_gm_spmv<View>, grid), KT, 0, st>>>(A, S, G, i, w1, Vk(0), w, part, ticket, grid);
+      k_gm_spmv<View><<<g1, KT, 0, st>>>(A, S, G, i, w1, Vk(0), w, part, ticket, grid);
       for (int k = 2; k <= i; k++)
-        k_gm_mgs<<<resident_grid(k_gm_mgs, grid), KT, 0, st>>>(S, G, i, k, n, Vk(k - 2), Vk(k - 1), w, part, ticket, grid);
-      k_gm_norm<<<resident_grid(k_gm_norm, grid), KT, 0, st>>>(S, G, i, nl, n, Vk(i - 1), w, part, ticket, grid);
+        k_gm_mgs<<<gm, KT, 0, st>>>(S, G, i, k, n, Vk(k - 2), Vk(k - 1), w, part, ticket, grid);
+      k_gm_norm<<<gn, KT, 0, st>>>(S, G, i, nl, n, Vk(i - 1), w, part, ticket, grid);
       per_graph += 3 + (i - 1) + long_launch(A);
     }
     k_gm_trsm<<<1, 32, 0, st>>>(S, G);
@@ -2044,13 +2049,14 @@ static int solve_cgs(const View &A, const double *dinv, const double *b, double 
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) rc = psbx_cuda_status(e, "BeginCapture");
   if (!rc) {
+    const int g1 = resident_grid(k_cgs_spmv1<View>, grid), g2 = resident_grid(k_cgs_spmv2<View>, grid);
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       k_cgs_p<<<grid, KT, 0, st>>>(S, n, r, q, dinv, uv, p, f);
       psbx_long_rows(A, f, &S->status, st);
-      k_cgs_spmv1<View><<<resident_grid(k_cgs_spmv1<View>, grid), KT, 0, st>>>(A, S, f, rt, v, part, ticket, grid);
+      k_cgs_spmv1<View><<<g1, KT, 0, st>>>(A, S, f, rt, v, part, ticket, grid);
       k_cgs_q<<<grid, KT, 0, st>>>(S, n, uv, v, dinv, q, z, x);
       psbx_long_rows(A, z, &S->status, st);
-      k_cgs_spmv2<View><<<resident_grid(k_cgs_spmv2<View>, grid), KT, 0, st>>>(A, S, z, rt, x, r, part, ticket, grid);
+      k_cgs_spmv2<View><<<g2, KT, 0, st>>>(A, S, z, rt, x, r, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");
@@ -2238,12 +2244,13 @@ static int solve_bicg(const View &A, void *mat, int fmt, const double *dinv, con
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) rc = psbx_cuda_status(e, "BeginCapture");
   if (!rc) {
+    const int g1 = resident_grid(k_bicg_spmv<View>, grid), gu = resident_grid(k_bicg_update, grid);
     for (int k = 0; k < KGRAPH_ITERS; k++) {
       k_bicg_p<<<grid, KT, 0, st>>>(S, n, z, zt, p, pt);
       psbx_long_rows(A, p, &S->status, st);
-      k_bicg_spmv<View><<<resident_grid(k_bicg_spmv<View>, grid), KT, 0, st>>>(A, S, p, pt, q, part, ticket, grid);
+      k_bicg_spmv<View><<<g1, KT, 0, st>>>(A, S, p, pt, q, part, ticket, grid);
       k_spmv_t<<<grid, KT, 0, st>>>(S, n, tirp, tja, tval, pt, qt);
-      k_bicg_update<<<resident_grid(k_bicg_update, grid), KT, 0, st>>>(S, n, p, q, qt, dinv, x, r, rt, z, zt, part, ticket, grid);
+      k_bicg_update<<<gu, KT, 0, st>>>(S, n, p, q, qt, dinv, x, r, rt, z, zt, part, ticket, grid);
     }
     e = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess) rc = psbx_cuda_status(e, "EndCapture");
