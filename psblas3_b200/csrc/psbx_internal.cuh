@@ -359,7 +359,18 @@ __device__ __forceinline__ void final_sum_dd(const double *part, int stride, int
     out[k] = dd_t{0.0, 0.0};
   }
   // four blocks' pairs in flight at once: the reads of one block's finaliser
-  // are the tail of every reducing kernel
+  // are the tail of every reducing kernel; a pair per thread when that is all
+  if (n <= (int)blockDim.x) {
+    if ((int)threadIdx.x < n) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const double2 t = __ldcg((const double2 *)part + (size_t)k * stride + threadIdx.x);
+        out[k] = dd_merge(out[k], dd_t{t.x, t.y});
+      }
+    }
+    block_sum_dd<NV>(out, smem);
+    return;
+  }
   for (int i = threadIdx.x; i < n; i += 4 * blockDim.x) {
     dd_t u[4][NV];
 #pragma unroll
