@@ -50,8 +50,8 @@ enum { BT = 256, ITERS = 8, MAXK = 8, LONG_ROW = 64 };
 // 86 ms a solve of all with 4096 rows, 69 with 2048, 60 with 1024, 66 with 512;
 // 128 anisotropic systems with eight: 390 ms with 2048, 320 with 1024, 336
 // with 512 (16 of them: 91, 61, 62).
-__host__ __device__ constexpr int tile_rows(int /*K*/) { return 1024; }
-__host__ __device__ constexpr int tile_nnz(int K) { return 8 * tile_rows(K); }
+// (one bound for both, so a matrix has one plan for every engine)
+enum { TILE_ROWS = 1024, TILE_NNZ = 8 * TILE_ROWS };
 
 // Eight right-hand sides are spread over L = 2 neighbouring lanes of H = 4
 // each: a row of a vector is then one 16-byte (FP32) access per lane, a warp
@@ -467,7 +467,7 @@ template <int K, int NS> struct TileSums {
   static constexpr int H = Lay<K>::H;
   static_assert(K == 1 || Lay<K>::R == CLS, "a thread's rows are CLS apart");
   struct Shared {
-    double term[K == 1 ? NS : 1][K == 1 ? tile_rows(K) : 1];
+    double term[K == 1 ? NS : 1][K == 1 ? TILE_ROWS : 1];
     double group[2][NS * K][GROUPS];  // two tiles in turn
   };
   Shared &sh;
@@ -493,7 +493,7 @@ template <int K, int NS> struct TileSums {
       if (m < NS) {  // whole warps
         double t = 0.0;
 #pragma unroll
-        for (int u = 0; u < tile_rows(K) / CLS; u++)
+        for (int u = 0; u < TILE_ROWS / CLS; u++)
           if (c + u * CLS < n) t = radd(t, sh.term[m][c + u * CLS]);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) t = radd(t, __shfl_down_sync(0xffffffffu, t, o));
@@ -1109,15 +1109,13 @@ static void capture_iters(Eng *e, cudaStream_t st) {
 // row lengths and kept on the matrix (the arrays' rewrite drops it): runs of
 // up to BT/32 consecutive rows longer than LONG_ROW become long-row
 // tiles; the rows between them are cut into thread-per-row tiles of at most
-// tile_rows(K) rows and tile_nnz(K) stored entries -- whole passes of the block
+// TILE_ROWS rows and TILE_NNZ stored entries -- whole passes of the block
 // where the entry bound cuts -- so no thread carries a long serial chain
 // (the head of a row-sorted power-law matrix, a long row among short ones).
 // It depends on the matrix alone, so a system's tiles and the order of its
-// partial sums do not depend on the other systems in the engine (the plan is
-// rebuilt when an engine with another K adds the matrix).
-static int tile_plan(HllDevice *m, int K) {
+// partial sums do not depend on the engine or the other systems in it.
+static int tile_plan(HllDevice *m) {
   const int n = m->rows;
-  const int trows = tile_rows(K), tnnz = tile_nnz(K);
   std::vector<int> irn(n > 0 ? n : 1);
   if (n > 0) PSBX_CK(cudaMemcpy(irn.data(), m->rS, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
   std::vector<int> plan;
@@ -1128,8 +1126,8 @@ static int tile_plan(HllDevice *m, int K) {
       plan.insert(plan.end(), {r, e - r, 1});
     } else {
       long long ent = 0;
-      while (e < n && e - r < trows && irn[e] <= LONG_ROW && ent + irn[e] <= tnnz) ent += irn[e++];
-      const bool entry_cut = e < n && e - r < trows && irn[e] <= LONG_ROW;
+      while (e < n && e - r < TILE_ROWS && irn[e] <= LONG_ROW && ent + irn[e] <= TILE_NNZ) ent += irn[e++];
+      const bool entry_cut = e < n && e - r < TILE_ROWS && irn[e] <= LONG_ROW;
       if (entry_cut && e - r > BT) e = r + (e - r) / BT * BT;
       plan.insert(plan.end(), {r, e - r, 0});
     }
@@ -1141,7 +1139,6 @@ static int tile_plan(HllDevice *m, int K) {
   free(m->tplan);
   m->tplan = t;
   m->ntplan = (int)(plan.size() / 3);
-  m->tplanK = K;
   return SPGPU_SUCCESS;
 }
 
@@ -1225,7 +1222,7 @@ int psbx_batch_create_prec(void **eng, int max_systems, int max_rows_total, int 
   e->K = nrhs;
   e->fp64 = inner_bits == 64;
   e->max_sys = max_systems;
-  e->max_tiles = max_rows_total / tile_rows(e->K) + max_systems + 1;
+  e->max_tiles = max_rows_total / TILE_ROWS + max_systems + 1;
   e->sms = c.sms;
   e->h_sys.assign(max_systems, BSys());
   e->h_state.assign(max_systems, BState());
@@ -1303,8 +1300,8 @@ int psbx_batch_add(void *eng, void *hllMat, const double *d_b, double *d_x, cons
       break;
     }
   if (s < 0) return SPGPU_OUTOFMEMORY;  // no free slot
-  if (!m->tplan || m->tplanK != e->K) {
-    int rc = tile_plan(m, e->K);
+  if (!m->tplan) {
+    int rc = tile_plan(m);
     if (rc) return rc;
   }
   PsbxCtx &c = psbx_ctx();

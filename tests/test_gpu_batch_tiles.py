@@ -66,3 +66,33 @@ def test_tile_edges(psb, nrhs, fp64):
         assert rel.max() <= 1.01e-10  # the engine's own residual, summed in another order
     for i in (8, 9, 11, 12):
         assert np.array_equal(solve([i])[i], res[i])
+
+
+def test_one_plan_for_both_engines(psb):
+    """A matrix that engines of one and of eight right-hand sides add in turn
+    (one tile plan, built once): the same bits every time, and each column of
+    eight equals the solve of that column alone."""
+    import torch
+    irp, ja, va = gen.powerlaw_spd(2300, kmax=40, seed=6)
+    n = len(irp) - 1
+    assert np.diff(irp).max() <= 64  # longer rows are summed in another way for eight
+    A, P = _hll(psb, irp, ja, va)
+    b = np.random.default_rng(2).uniform(-1, 1, (n, 8))
+
+    def solve(nrhs, cols):
+        eng = psb.BatchSolver(1, n, nrhs)
+        d = torch.from_numpy(np.ascontiguousarray(cols).reshape(-1)).cuda()
+        x = torch.zeros_like(d)
+        torch.cuda.synchronize()
+        slot = eng.add(A, d, x, P.dv.data_ptr, eps=1e-10)
+        eng.run(replays_per_step=2)
+        assert eng.poll(slot)[0] == 1
+        res = x.cpu().numpy().reshape(n, nrhs)
+        eng.free()
+        return res
+
+    one = solve(1, b[:, :1])
+    eight = solve(8, b)
+    assert np.array_equal(solve(1, b[:, :1]), one)
+    assert np.array_equal(solve(8, b), eight)
+    assert np.array_equal(solve(1, b[:, 5:6])[:, 0], eight[:, 5]) and np.array_equal(one[:, 0], eight[:, 0])
