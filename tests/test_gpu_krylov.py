@@ -12,6 +12,10 @@ from psblas3_b200 import gen
 
 pytestmark = pytest.mark.gpu
 
+# CG and BiCGSTAB of small systems run as one kernel up to an itmax of 100,000,
+# with a kernel per step above it
+BOTH = pytest.mark.parametrize("itmax", [1000, 200_000])
+
 
 def _mats(psb, irp, ja, va, fmt):
     n = len(irp) - 1
@@ -56,34 +60,38 @@ def test_bicgstab_c1(psb):
     assert np.max(np.abs(x - xo)) <= 1e-6
 
 
+@BOTH
 @pytest.mark.parametrize("fmt", ["HLL", "ELL", "CSR"])
 @pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
-def test_methods_formats_poisson(psb, fmt, method):
+def test_methods_formats_poisson(psb, fmt, method, itmax):
     irp, ja, va = gen.poisson7(24)
     n = len(irp) - 1
     b = np.random.default_rng(3).uniform(-1, 1, n)
-    (x, it, err), (xo, ito, erro) = _solve_both(psb, method, irp, ja, va, b, fmt=fmt, eps=1e-8)
+    (x, it, err), (xo, ito, erro) = _solve_both(psb, method, irp, ja, va, b, fmt=fmt, eps=1e-8, itmax=itmax)
     assert abs(it - ito) <= 2, (it, ito)
     assert err <= 1e-8
     r = b - gen.csr_matvec(irp, ja, va, x)
     assert np.linalg.norm(r) <= 2e-8 * np.linalg.norm(b)
 
 
+@BOTH
+@pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
 @pytest.mark.parametrize("istop", [1, 2, 3])
-def test_stop_criteria(psb, istop):
-    irp, ja, va = gen.pde3d(14, b=(0.5, 0.25, 0.0))
+def test_stop_criteria(psb, istop, method, itmax):
+    irp, ja, va = gen.pde3d(14, b=(0.5, 0.25, 0.0)) if method == "BICGSTAB" else gen.poisson7(14)
     n = len(irp) - 1
     b = np.random.default_rng(4).uniform(-1, 1, n)
-    (x, it, err), (xo, ito, erro) = _solve_both(psb, "BICGSTAB", irp, ja, va, b, eps=1e-7, istop=istop)
+    (x, it, err), (xo, ito, erro) = _solve_both(psb, method, irp, ja, va, b, eps=1e-7, istop=istop, itmax=itmax)
     assert abs(it - ito) <= 2, (istop, it, ito)
     assert err <= 1e-7
 
 
-def test_cg_no_prec_and_itmax(psb):
+@BOTH
+def test_cg_no_prec_and_itmax(psb, itmax):
     irp, ja, va = gen.poisson7(16)
     n = len(irp) - 1
     b = np.random.default_rng(5).uniform(-1, 1, n)
-    (x, it, err), (xo, ito, erro) = _solve_both(psb, "CG", irp, ja, va, b, prec=False, eps=1e-10)
+    (x, it, err), (xo, ito, erro) = _solve_both(psb, "CG", irp, ja, va, b, prec=False, eps=1e-10, itmax=itmax)
     assert abs(it - ito) <= 2
     # itmax stops the solve with iter == itmax, err above eps (as the reference)
     (x, it, err), (xo, ito, erro) = _solve_both(psb, "CG", irp, ja, va, b, eps=1e-14, itmax=7)
@@ -215,12 +223,14 @@ def test_bicgstabl_c1(psb, irst, istop):
     assert np.max(np.abs(x - xo)) <= 1e-8
 
 
+@BOTH
 @pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
-def test_repeated_solves_replay_kept_graph(psb, method):
-    """Calls with the same matrix view and vectors replay the iteration graph
-    kept from the first call: the same iterations, error and bits; new values
-    in the same right-hand side vector solve the new system; a nonzero
-    initial guess is honoured; another vector is another graph."""
+def test_repeated_solves_replay_kept_graph(psb, method, itmax):
+    """Calls with the same matrix view and vectors -- which replay the iteration
+    graph kept from the first call, or run the one kernel again: the same
+    iterations, error and bits; new values in the same right-hand side vector
+    solve the new system; a nonzero initial guess is honoured; another vector
+    is another graph."""
     irp, ja, va = gen.pde3d(14, a=(1, 1, 1), b=(1 / np.sqrt(3),) * 3) if method == "BICGSTAB" else gen.poisson7(14)
     n = len(irp) - 1
     import torch
@@ -233,26 +243,29 @@ def test_repeated_solves_replay_kept_graph(psb, method):
     runs = []
     for _ in range(3):
         X.zero()
-        it, err = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=2000)
+        l0 = psb.kernel_launches()
+        it, err = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=itmax)
+        assert (psb.kernel_launches() - l0 == 1) == (itmax <= 100_000)
         runs.append((it, err, X.get_vect()))
     for it, err, x in runs[1:]:
         assert it == runs[0][0] and err == runs[0][1] and np.array_equal(x, runs[0][2])
     B.set_vect(b2)
     X.set_vect(x0)
-    it, err = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=2000)
+    it, err = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=itmax)
     assert err <= 1e-10
     r = b2 - gen.csr_matvec(irp, ja, va, X.get_vect())
     assert np.linalg.norm(r) <= 1e-9 * np.linalg.norm(b2)
     # a second solution vector: its own graph, same answer as the first one's
     X2 = psb.DVect(n)
     X.zero()
-    it_a, err_a = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=2000)
-    it_b, err_b = psb.psb_krylov(method, A, P, B, X2, eps=1e-10, itmax=2000)
+    it_a, err_a = psb.psb_krylov(method, A, P, B, X, eps=1e-10, itmax=itmax)
+    it_b, err_b = psb.psb_krylov(method, A, P, B, X2, eps=1e-10, itmax=itmax)
     assert (it_a, err_a) == (it_b, err_b) and np.array_equal(X.get_vect(), X2.get_vect())
 
 
+@BOTH
 @pytest.mark.parametrize("fmt", ["HLL", "ELL", "CSR"])
-def test_random_systems_cg_bicgstab(psb, fmt):
+def test_random_systems_cg_bicgstab(psb, fmt, itmax):
     """Seeded random diagonally dominant systems (rows of 0 .. 12 random
     off-diagonal entries, the diagonal their absolute sum plus 1): CG on the
     symmetric ones (A + A^T), BiCGSTAB on the nonsymmetric ones, DIAG: the
@@ -277,7 +290,8 @@ def test_random_systems_cg_bicgstab(psb, fmt):
             fi, fj, fv = O.coo_fix(n, ii, jj, vv)
             irp, cja, cva = O.csr_from_coo(n, fi, fj, fv)
             b = rng.uniform(-1, 1, n)
-            (x, it, err), (xo, ito, erro) = _solve_both(psb, method, irp, cja, cva, b, fmt=fmt, eps=1e-9)
+            (x, it, err), (xo, ito, erro) = _solve_both(psb, method, irp, cja, cva, b, fmt=fmt, eps=1e-9,
+                                                        itmax=itmax)
             assert abs(it - ito) <= 2, (seed, method, it, ito)
             assert err <= 1e-9 and erro <= 1e-9
             assert np.max(np.abs(x - xo)) <= 1e-7 * max(1.0, np.max(np.abs(xo)))
