@@ -6,6 +6,7 @@ and those are compensated, so iterations and solutions agree."""
 import numpy as np
 import pytest
 
+import oracle as O
 from psblas3_b200 import gen
 
 pytestmark = pytest.mark.gpu
@@ -137,17 +138,57 @@ def test_uneven_rows_go_to_the_drivers(psb, fmt):
     assert _solve(psb, _matrix(psb, fmt, irp, ja, va), "CG", b[:66 ** 3], 5000)[3] == 1
 
 
+# 3 x 3 blocks whose solves break down exactly (small integers and powers of
+# two up to there) in the second iteration, x moved by the first, and converge
+# after the restart: matrix, right-hand side, x0
+_BREAKING = {
+    "CG": [([[2, 3, 0], [3, 3, 1], [0, 1, -1]], [0, -3, 2], [1, -1, -2]),
+           ([[-3, 1, 2], [1, -2, 0], [2, 0, -1]], [-3, 2, 1], [-1, -1, -2])],
+    "BICGSTAB": [([[2, 1, 3], [1, 2, 0], [-1, 1, 1]], [3, 3, 1], [-1, 2, -2]),
+                 ([[-3, -1, 1], [0, -2, 0], [3, 0, 0]], [3, 2, -2], [-2, 1, -2])],
+}
+
+
+@pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
+@pytest.mark.parametrize("which", [0, 1])
+@pytest.mark.parametrize("copies", [1, 1500, 7000])
+def test_restart_after_breakdown(psb, method, which, copies):
+    """A breakdown with x past x0: each block stores its rows of x, and the
+    restart's product reads the rows of other blocks (the three rows of a
+    system are `copies` apart).  One block, blocks up to 64 and beyond; as the
+    oracle and the kernel-per-step drivers."""
+    import scipy.sparse as sp
+    a, b, x0 = _BREAKING[method][which]
+    m = sp.kron(sp.csr_matrix(np.array(a, float)), sp.identity(copies)).tocsr()
+    m.eliminate_zeros()
+    m.sort_indices()
+    irp, ja, va = (m.indptr + 1).astype(np.int32), (m.indices + 1).astype(np.int32), m.data
+    b, x0 = (np.repeat(np.array(v, float), copies) for v in (b, x0))
+    xo, ito, _ = O.krylov(method, irp, ja, va, b, x0=x0, eps=1e-10, itmax=40)
+    assert ito == 5  # two iterations, the restart, three more
+    A = _matrix(psb, "CSR", irp, ja, va)
+    for itmax in (40, GENERAL):
+        it, err, x, launches = _solve(psb, A, method, b, itmax, prec=False, x0=x0)
+        assert (launches == 1) == (itmax == 40)
+        assert it == ito and err <= 1e-10
+        assert np.max(np.abs(x - xo)) <= 1e-9 * max(1.0, np.max(np.abs(xo)))
+
+
 @pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
 def test_breakdown_and_itmax(psb, method):
-    """A breakdown at every restart ends at itmax, as in the general path; so
-    does a solve that does not converge, and b = 0."""
+    """A breakdown at every restart ends at itmax with x untouched, as in the
+    oracle; a solve that does not converge ends there too, and b = 0 at once
+    or by breakdowns."""
     irp, ja, va = np.array([1, 2, 3], np.int32), np.array([2, 1], np.int32), np.array([1.0, 1.0])
     A = _matrix(psb, "CSR", irp, ja, va)
-    it, _, _, _ = _solve(psb, A, method, np.array([1.0, 0.0]), 7, prec=False)
-    assert it <= 7
+    b = np.array([1.0, 0.0])
+    xo, ito, _ = O.krylov(method, irp, ja, va, b, itmax=7)
+    it, _, x, launches = _solve(psb, A, method, b, 7, prec=False)
+    assert launches == 1 and it == ito == 7 and np.array_equal(x, xo)
     irp, ja, va = gen.poisson7(12)
     A = _matrix(psb, "HLL", irp, ja, va)
     it, err, _, launches = _solve(psb, A, method, np.random.default_rng(0).uniform(-1, 1, 1728), 5)
     assert it == 5 and err > 1e-10 and launches == 1
+    _, ito, _ = O.krylov(method, irp, ja, va, np.zeros(1728), itmax=9)
     it, err, x, _ = _solve(psb, A, method, np.zeros(1728), 9)
-    assert not x.any()
+    assert it == ito and not x.any()
