@@ -15,6 +15,10 @@
 //   reach the number of blocks, then warp 0 reads all slots.  With 148 blocks
 //   polling 148 slots the polls hold up the late stores: 3.7 us against 2.9 us
 //   (measured in the solver's loop, two sums).
+// The line between them, us an iteration of CG and of BiCGSTAB with tags and with
+// the counter: 9 blocks 5.7 / 6.6 and 9.9 / 11.2; 32 6.6 / 6.8 and 11.4 / 11.5; 42
+// 6.75 / 6.82 and 11.5 / 11.4; 48 6.85 / 6.82 and 11.7 / 11.4; 62 7.0 / 6.8 and
+// 12.0 / 11.4; 148 13.0 / 11.0 and 23.7 / 19.7.
 //
 // Two slot buffers alternate: a block publishes reduction s + 2 only after it
 // has seen every block's s + 1, which a block publishes after it has read all
@@ -42,7 +46,7 @@ struct GridSync {
   int nblocks;
 };
 #define GS_SLOT 8                        // 16-byte words of a slot
-#define GS_TAG_BLOCKS 64
+#define GS_TAG_BLOCKS 40
 #define GS_MAXB 160                      // blocks of a launch: one per SM
 #define GS_BYTES(nblocks) (sizeof(ulonglong2) * GS_SLOT * (2 * (size_t)(nblocks) + 2))
 
@@ -221,7 +225,9 @@ __device__ __forceinline__ void grid_reduce(GridSync &g, dd_t (&s)[S > 0 ? S : 1
   for (int k = 0; k < S; k++) s[k] = dd_t{0.0, 0.0};
 #pragma unroll
   for (int k = 0; k < M; k++) m[k] = 0.0;
-  // slots t, t + blockDim, ... by thread t, in block order within a thread.
+  // slots t, t + blockDim, ... by thread t, in block order within a thread (one
+  // slot as GS_TAG_BLOCKS stands; written without the loop, the solver's
+  // registers come out 3 to 6 % slower).
   // The lanes of a warp leave the wait together, those without a slot too:
   // with some lanes ahead at the shuffles below, a reduction took 7 us.
   const int nread = np < nw ? np : nw;  // warps that read slots

@@ -72,12 +72,12 @@ def _agree(psb, A, method, b, **kw):
 
 
 @pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 256, 257, 4100, 20001, 75777])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 256, 257, 4100, 10240, 10241, 20001, 75777])
 def test_sizes(psb, method, n):
     """One row to more rows than threads: partial slices, one and many blocks
-    (both ways of publishing a reduction), several slices per warp.  (On one
-    or two rows BiCGSTAB breaks down before its first update of x, in every
-    restart.)"""
+    (both ways of publishing a reduction, with 40 and 41 blocks at the line),
+    several slices per warp.  (On one or two rows BiCGSTAB breaks down before
+    its first update of x, in every restart.)"""
     if method == "BICGSTAB" and n < 3:
         n = 3
     irp, ja, va = gen.powerlaw(n, kmax=min(6, n - 1), seed=n) if n > 2 else _dominant(n, n)
