@@ -456,10 +456,13 @@ __device__ __forceinline__ void tile_spmv(const BSys &S, const BTile &T, const V
   }
 }
 
-// NS sums over a tile's rows per rhs, in one order whatever K is, so that a
-// right-hand side gives the same bits alone and among eight: the terms of
-// rows c, c + 128, c + 256, ... in order, for each c < 128; 16 neighbouring c
-// in a tree; the 8 groups in order.  With eight right-hand sides those rows
+// NS sums over a tile's rows per rhs; in thread-per-row tiles in one order
+// whatever K is, so that a right-hand side gives the same bits alone and among
+// eight: the terms of rows c, c + 128, c + 256, ... in order, for each c < 128;
+// 16 neighbouring c in a tree; the 8 groups in order.  (Not so for rows longer
+// than LONG_ROW: the block and the warp that sum such a row for one and for
+// eight right-hand sides add its entries in other orders, and their terms fall
+// into other classes.)  With eight right-hand sides those rows
 // are one thread's, which keeps its sums in registers; with one, a pass of the
 // block is two of these rows, and the terms go to shared memory first.
 enum { CLS = 128, GROUPS = CLS / 16 };
