@@ -99,3 +99,32 @@ def test_forms_at_grid_lines(psb, blocks, longest):
         X, Y = psb.DVect.bld(x32), psb.DVect.bld(y32)
         A.spmv(-0.5, X, 2.0, Y)
         assert np.array_equal(Y.get_vect(), ref32)
+
+
+@pytest.mark.parametrize("longest", [1, 3, 8, 17, 23, 24, 29])
+@pytest.mark.parametrize("n", [33, 160_001])
+def test_ell_float_forms(psb, n, longest):
+    """FP32 ELL rows on either side of the line at 24 entries: the FP64 row sum
+    rounded once."""
+    import ctypes as C
+    from psblas3_b200._lib import lib
+    irp, ja, va = _bands(n, longest, 3)
+    irn = np.diff(irp).astype(np.int32)
+    h = C.c_void_p()
+    assert lib.FallocEllDevice(C.byref(h), n, longest, len(ja), n, 1, 1) == 0
+    pitch = lib.getEllDevicePitch(h)
+    rows = np.repeat(np.arange(n), irn)
+    at = (np.arange(len(ja)) - np.repeat(irp[:-1] - 1, irn)) * pitch + rows
+    eja, eva = np.ones(pitch * longest, np.int32), np.zeros(pitch * longest, np.float32)
+    eja[at], eva[at] = ja, va
+    ptr = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    assert lib.writeEllDeviceFloat(h, ptr(eva), ptr(eja), pitch, ptr(irn), ptr(np.zeros(n, np.int32))) == 0
+    x, y0 = np.random.default_rng(4).uniform(-1, 1, (2, n)).astype(np.float32)
+    s = O.csr_csmv(irp, ja, va.astype(np.float32).astype(np.float64), 1.0, x.astype(np.float64), 0.0,
+                   np.zeros(n)).astype(np.float32)
+    for alpha, beta in ((1.0, 0.0), (-0.5, 2.0)):
+        X, Y = psb.DVect.bld(x), psb.DVect.bld(y0)
+        assert lib.spmvEllDeviceFloat(h, np.float32(alpha), X.h, np.float32(beta), Y.h) == 0
+        ref = np.float32(alpha) * s
+        assert np.array_equal(Y.get_vect(), ref if beta == 0.0 else ref + np.float32(beta) * y0)
+    lib.freeEllDevice(h)
